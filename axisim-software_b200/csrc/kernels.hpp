@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "device.cuh"
 
 namespace axisim {
@@ -92,6 +94,64 @@ struct ResidentArgsT {
     MgOp ops[kMaxResidentOps];
     TailArgsT<T> tail;
     size_t smem = 0;  // dynamic shared memory the phases need
+};
+
+// The deep levels of a V-cycle in one launch of one thread-block cluster
+// (mg_cluster.cu), levels first .. first + count - 1: levels of at most
+// kClusterSolo cells on CTA 0, larger ones in chunks of rows on the other CTAs
+// (a single CTA where every level is solo).
+constexpr int kClusterSize = 16;
+constexpr int kMaxClusterLevels = 10;
+constexpr int kClusterMaxCells = 15 * 1024;
+constexpr int kClusterSolo = 1024;
+constexpr size_t kClusterMaxShared = 220 * 1024;
+// A level on one CTA: its rows from global cell row0, and offsets into the
+// CTA's shared memory. Cells are numbered rows, halo, padding, zero cell.
+struct ClusterRows {
+    int32_t rows = 0, row0 = 0, live = 0, cells = 0;  // live: rows and halo
+    int32_t wide = 0;             // a slice has more than eight slots a row: `so` holds slot base | groups << 24
+    int32_t slot0 = 0, slots = 0;  // this CTA's run of the level's slots
+    uint32_t nb = 0, so = 0, halo = 0, c2c = 0, ms = 0, ml = 0;
+    uint32_t value64 = 0, value32 = 0;  // the level's values, by precision
+};
+struct MgClusterPlan {
+    int first = -1, count = 0, ctas = 0;
+    uint32_t blobBytes = 0;               // per CTA
+    const unsigned char* blob = nullptr;  // device, one block per CTA: its ClusterRows, then what they point to
+    size_t shared64 = 0, shared32 = 0;
+    int32_t W[kMaxClusterLevels] = {};
+    bool solo[kMaxClusterLevels] = {};
+};
+enum ClusterOp : uint8_t { kClSweep, kClResidual, kClRestrict, kClCorrect, kClHalo, kClCoarsest, kClStore };
+struct ClusterStep {
+    void* global = nullptr;   // the values in L2 that the step reads or writes
+    void* global2 = nullptr;
+    ClusterOp op = kClSweep;
+    uint8_t level = 0, from = 0, to = 0, clusterWide = 0;
+    int32_t flag = 0;
+};
+constexpr int kMaxClusterSteps = 64;
+struct GridLevel;
+// The plan of levels first.. and the packed topology of its CTAs; false when
+// they do not fit (a level above kClusterMaxCells, too many levels, shared
+// memory). sliceOff, mStart, mList: the levels' slice offsets and member lists.
+bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::vector<std::vector<int32_t>>& sliceOff,
+                      const std::vector<std::vector<int32_t>>& mStart, const std::vector<std::vector<int32_t>>& mList,
+                      MgClusterPlan& plan, std::vector<unsigned char>& blob);
+bool clusterRunnable(const MgClusterPlan& plan);
+template <class T>
+struct ClusterArgsT {
+    MgClusterPlan plan;
+    const T* AF[kMaxClusterLevels] = {};
+    const T* AC[kMaxClusterLevels] = {};
+    T* x[kMaxClusterLevels][2] = {};  // level `first`: x[0] is the iterate, in and out
+    T* res[kMaxClusterLevels] = {};
+    const T* b = nullptr;  // level `first`
+    T w = T(0.6), scale = T(1);
+    int pre = 1, post = 1, coarse = 30;
+    int firstDone = 0;  // the iterate already holds the first pre-smoothing sweep
+    int nSteps = 0, syncFirst = 0;  // filled by the launch
+    ClusterStep steps[kMaxClusterSteps];
 };
 
 // ---- setup ----
@@ -230,6 +290,9 @@ void launchMGTerminal(const Ctl* ctl, const LevelT<T>& L, T* x, T w, int sweeps,
 // device cannot hold the grid or the program does not fit
 template <class T>
 bool launchMGResident(Ctl* ctl, const ResidentArgsT<T>& a, cudaStream_t s);
+// the levels of a.plan as one cluster launch; false when it cannot run
+template <class T>
+bool launchMGCluster(const Ctl* ctl, ClusterArgsT<T> a, cudaStream_t s);
 template <class T>
 size_t tailSharedBytes(const TailArgsT<T>& a);
 template <class T>

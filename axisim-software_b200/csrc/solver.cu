@@ -1207,6 +1207,7 @@ private:
                     int w = 0;
                     for (int c = sI * 32; c < std::min(g.nCells, sI * 32 + 32); c++)
                         w = std::max(w, g.faceStart[(size_t)c + 1] - g.faceStart[(size_t)c]);
+                    if (g.nCells <= kClusterMaxCells) w = (w + 7) & ~7;  // groups of eight slots (mg_cluster.cu)
                     off[(size_t)sI + 1] = off[(size_t)sI] + 32 * w;
                     W = std::max(W, w);
                 }
@@ -1231,6 +1232,7 @@ private:
                 d.res = mgArena_.alloc<double>((size_t)g.nCells);
             }
         }
+        std::vector<std::vector<int32_t>> mStartH((size_t)L), mListH((size_t)L);
         for (int l = 1; l < L; l++) {
             const GridLevel& f = hier_[(size_t)l - 1];
             const GridLevel& c = hier_[(size_t)l];
@@ -1292,6 +1294,8 @@ private:
             cd.gStart = mgArena_.upload(gStart.data(), gStart.size());
             cd.gList = mgArena_.upload(gList.data(), gList.size());
             fd.internalMask = mgArena_.upload(mask.data(), mask.size());
+            mStartH[(size_t)l] = std::move(mStart);
+            mListH[(size_t)l] = std::move(mList);
         }
         int lastTerminal = -1;
         for (int l = 0; l < (int)termRanges_.size() && l < L; l++) {
@@ -1319,8 +1323,20 @@ private:
                 break;
             }
         }
+        // the finest level from which on all fit one thread-block cluster
+        cluster_ = MgClusterPlan();
+        for (int t = std::max(1, lastTerminal + 1); t < L; t++) {
+            MgClusterPlan plan;
+            std::vector<unsigned char> blob;
+            if (!buildClusterPlan(hier_, t, sliceOffH, mStartH, mListH, plan, blob)) continue;
+            if (!clusterRunnable(plan)) break;
+            plan.blob = mgArena_.upload(blob.data(), blob.size());
+            cluster_ = plan;
+            break;
+        }
     }
     int tailStart_ = -1;
+    MgClusterPlan cluster_;  // first < 0: none
     bool galerkinThisSolve_ = true;  // false: the coarse operators of this p' solve are already built
     double* irUpdate_ = nullptr;     // set during a mixed refinement cycle: the FP64 iterate it corrects
     bool irUpdated_ = false;         // the cycle's last finest-level pass applied the correction
@@ -1536,6 +1552,7 @@ private:
         const T w = (T)cmg_.weight;
         const char* tag = sizeof(T) == 8 ? "" : "32";
         const double vb = (double)sizeof(T);
+        if (l == cluster_.first && !residentVcycle_ && clusterCycle<T>(lv, cur, alt, firstDone)) return;
         if (hier_[(size_t)l].isCoarsest()) {
             smoothT<T>(lv, l, cmg_.linearSweep - (firstDone ? 1 : 0), cur, alt);
             return;
@@ -1547,7 +1564,8 @@ private:
         // itself (one launch instead of two where launches dominate); larger
         // levels, the finest one (coalesced [W][N] rows) and the level above
         // the tail (whose residual the tail reads) keep the separate pass
-        const bool gatherRes = F.sliceOff != nullptr && F.N <= kFuseMaxCells && l + 1 != tailStart_;
+        const bool tail = l + 1 == tailStart_ && (l + 1 != cluster_.first || residentVcycle_);
+        const bool gatherRes = F.sliceOff != nullptr && F.N <= kFuseMaxCells && !tail;
         if (!gatherRes) {
             T* x = cur[(size_t)l];
             emit<T>(kOpResidual, l, x, nullptr, 0, 0.0, 0, std::string("mg_residual") + tag,
@@ -1556,8 +1574,8 @@ private:
         }
         // level l + 1's operator is read from here on; the tail reads every
         // level below it as well
-        joinGalerkin(l + 1 == tailStart_ ? L - 1 : l + 1);
-        if (l + 1 == tailStart_) {
+        joinGalerkin(tail || l + 1 == cluster_.first ? L - 1 : l + 1);
+        if (tail) {
             TailArgsT<T> a;
             a.first = l + 1;
             a.count = L - (l + 1);
@@ -1670,6 +1688,37 @@ private:
                     (4.0 + 2 * vb) * F.N + vb * C.N, [&] { launchMGProlong<T>(ctl_, F, x, xc, sc, stream_); });
             smoothT<T>(lv, l, post, cur, alt);
         }
+    }
+
+    // The cycle from the cluster's finest level down as one launch (in place in cur).
+    template <class T>
+    bool clusterCycle(std::vector<LevelT<T>>& lv, std::vector<T*>& cur, std::vector<T*>& alt, bool firstDone) {
+        ClusterArgsT<T> a;
+        a.plan = cluster_;
+        double bytes = 0.0;
+        for (int i = 0; i < cluster_.count; i++) {
+            const LevelT<T>& l = lv[(size_t)(cluster_.first + i)];
+            a.AF[i] = l.AF;
+            a.AC[i] = l.AC;
+            a.x[i][0] = l.x;
+            a.x[i][1] = l.xNew;
+            a.res[i] = l.res;
+            bytes += (double)l.totalSlots * (2.0 + sizeof(T)) + (double)l.N * sizeof(T);
+        }
+        const LevelT<T>& top = lv[(size_t)cluster_.first];
+        a.b = top.b;
+        a.x[0][0] = cur[(size_t)cluster_.first];
+        a.x[0][1] = alt[(size_t)cluster_.first];
+        a.w = (T)cmg_.weight;
+        a.scale = (T)curProlong_;
+        a.pre = cmg_.linearPreSweep;
+        a.post = cmg_.linearPostSweep;
+        a.coarse = cmg_.linearSweep;
+        a.firstDone = firstDone ? 1 : 0;
+        if (!launchMGCluster<T>(ctl_, a, stream_)) return false;
+        markL(std::string("mg_smooth_cluster") + (sizeof(T) == 8 ? "" : "32"), cluster_.first,
+              bytes + 3.0 * sizeof(T) * top.N);
+        return true;
     }
 
     // After level l's operator on galStream_: the event the V-cycle waits for.
