@@ -18,6 +18,7 @@
 // inner cycles of the mixed-precision path.
 #include <cmath>
 
+#include "coarsest.cuh"
 #include "kernels.hpp"
 
 namespace axisim {
@@ -226,6 +227,29 @@ __device__ __forceinline__ void terminalBody(const LevelT<T>& L, T* x, T w, int 
     const int s0 = L.term[2 * r], n1 = L.term[2 * r + 1];
     const int m = n1 - s0;
     T* xo = reinterpret_cast<T*>(smraw);
+    if (L.W <= 8 && m <= (int)blockDim.x && m > 0) {  // a row per thread, in registers
+        const int i = min((int)threadIdx.x, m - 1), n = s0 + i;
+        const Slots sl = slotsOf(L, n);
+        T c[8];
+        uint32_t adr[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int p = sl.base + min(j, max(sl.width - 1, 0)) * sl.stride;
+            const int k = j < sl.width ? L.nb[p] : -1;
+            c[j] = k >= 0 ? L.AF[p] : T(0);
+            adr[j] = (uint32_t)((k >= 0 ? k - s0 : m) * (int)sizeof(T));
+        }
+        const T ac = L.AC[n], bn = L.b[n];
+        for (int q = threadIdx.x; q <= m; q += blockDim.x) {
+            xo[q] = q < m ? T(0) : T(-0.0);  // the last cell: what unused slots read
+            xo[m + 1 + q] = xo[q];
+        }
+        __syncthreads();
+        coarsestSweeps<T>(smraw, 0, (uint32_t)((m + 1) * (int)sizeof(T)), (uint32_t)(i * (int)sizeof(T)), c, adr, ac, bn,
+                          (int)threadIdx.x < m, w, sweeps, [] { __syncthreads(); });
+        if ((int)threadIdx.x < m) x[n] = xo[(sweeps & 1) ? m + 1 + i : i];
+        return;
+    }
     T* xn = xo + m;
     for (int i = threadIdx.x; i < m; i += blockDim.x) xo[i] = T(0);
     __syncthreads();
@@ -909,7 +933,7 @@ void launchMGTerminal(const Ctl* ctl, const LevelT<T>& L, T* x, T w, int sweeps,
         configured = true;
     }
     const int threads = L.termMax < 256 ? ((L.termMax + 31) / 32) * 32 : 256;
-    launchPDL(k_mg_terminal<T>, dim3(L.nTerm), dim3(threads), 2 * (size_t)L.termMax * sizeof(T), s, ctl, L, x, w,
+    launchPDL(k_mg_terminal<T>, dim3(L.nTerm), dim3(threads), 2 * ((size_t)L.termMax + 1) * sizeof(T), s, ctl, L, x, w,
               sweeps);
 }
 

@@ -35,7 +35,7 @@
 
 #include <cooperative_groups.h>
 
-#include "exact_div.cuh"
+#include "coarsest.cuh"
 #include "host_prep.hpp"
 #include "kernels.hpp"
 
@@ -195,11 +195,7 @@ __device__ __forceinline__ void partSync(int threads) {
     else asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
-// The coarsest level's sweeps, one row per thread: coefficients, neighbour
-// addresses and the row's own value in registers, the quotient by the row's
-// diagonal from its reciprocal (exact_div.cuh), and only the warps that hold
-// rows in the barrier. What is left of a sweep is one shared-memory read, the
-// ordered sum and the quotient.
+// The coarsest level's sweeps (coarsest.cuh); only the warps that hold rows take part.
 template <class T>
 __device__ __forceinline__ void coarsestRows(const View<T>& L, uint32_t x, uint32_t y, T w, int sweeps, int part) {
     const int n = min((int)threadIdx.x, L.l.rows - 1);  // a surplus lane repeats the last row and stores nothing
@@ -212,24 +208,8 @@ __device__ __forceinline__ void coarsestRows(const View<T>& L, uint32_t x, uint3
         c[j] = at<T>(L.AF + (uint32_t)sizeof(T) * (s0 + 32 * j));
         adr[j] = x + at<uint16_t>(L.l.nb + 2 * (s0 + 32 * j)) * (uint32_t)sizeof(T);
     }
-    const T ac = at<T>(L.AC + o), bn = at<T>(L.b + o);
-    T xn = at<T>(x + o);
-    const bool empty = fabs(ac) < tinyOf<T>();
-    const ExactDiv<T> byAc(empty ? T(1) : ac);
-    const uint32_t flip = y - x;
-    uint32_t from = 0;
-    for (int it = 0; it < sweeps; it++) {
-        T g[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) g[j] = at<T>(adr[j] + from);
-        T Ax = ac * xn;
-#pragma unroll
-        for (int j = 0; j < 8; j++) Ax += c[j] * g[j];
-        xn = empty ? xn : xn + byAc(w * (bn - Ax));
-        from = flip - from;
-        if (live) at<T>(x + o + from) = xn;
-        partSync(part);
-    }
+    coarsestSweeps<T>(smraw, x, y, o, c, adr, at<T>(L.AC + o), at<T>(L.b + o), live, w, sweeps,
+                      [&] { partSync(part); });
 }
 
 template <class T>

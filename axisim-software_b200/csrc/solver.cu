@@ -1619,7 +1619,7 @@ private:
             if (C.nTerm > 0) {  // the cases whose coarsest level this is: their coarsest-level sweeps
                 T* x = cur[(size_t)l + 1];
                 const int sw = cmg_.linearSweep;
-                emit<T>(kOpTerminal, l + 1, x, nullptr, sw, 0.0, 2 * (size_t)C.termMax * sizeof(T),
+                emit<T>(kOpTerminal, l + 1, x, nullptr, sw, 0.0, 2 * ((size_t)C.termMax + 1) * sizeof(T),
                         std::string("mg_terminal") + tag, (double)C.N * ((4.0 + vb) * C.W + 3.0 * vb),
                         [&] { launchMGTerminal<T>(ctl_, C, x, w, sw, stream_); });
             }
