@@ -15,11 +15,14 @@
 // rows (dW, db, the loss) run as per-block partials summed in a fixed order,
 // so a training step is deterministic.
 //
-// The dense products are small (K <= 256 inputs, <= 128 outputs per row) and
-// run on the FP32 pipes with BF16 storage: at the finest level, where nearly
-// all rows are, a layer moves ~100 bytes and does ~1 kFLOP per row, far below
-// the ridge point of either the FP32 pipes or the tensor cores, so the layer is
-// bound by memory traffic, not by the multiply-adds.
+// The dense products are small (K <= 256 inputs, <= 128 outputs per row): at
+// the finest level, where nearly all rows are, a layer moves ~130 bytes and
+// does ~1 kFLOP per row, and the coarse levels have a few dozen to a few
+// thousand rows. So the finest levels are bound by memory traffic and the
+// coarse ones by the latency of one tile; the products run as mma.sync on
+// operands that go from global memory straight into fragments
+// (k_layer_mma, k_layer_dz_mma; BF16 weights) or through shared-memory tiles
+// (k_layer_tile, k_layer_dz_tile; FP32 weights, the gradient check's mode).
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -495,6 +498,357 @@ __global__ void __launch_bounds__(256) k_layer_dz_tile(NetLayer L, const TW* __r
     }
 }
 
+// ---------------- BF16 weights: fragments straight from memory ----------------
+//
+// A warp computes 16 rows times 8 NB columns of A B with mma.sync m16n8k16
+// (BF16 operands, FP32 accumulators) without staging A in shared memory. The
+// order of the inner index is free as long as A and B agree, so the lane that
+// holds k = 2t, 2t+1, 2t+8, 2t+9 of a fragment (t = lane % 4) takes the
+// channels 4t .. 4t+3 of each 16-channel slab: one 16-byte load per row and
+// slab, the four lanes of a row reading 64 consecutive bytes. B (the layer's
+// weights) is packed in that order when the weights change (k_pack), so a CTA
+// copies it as it is and a lane reads its four values of a column as 8 bytes.
+//
+// The FP32 operand A goes in as three BF16 parts, a = a1 + a2 + a3 with each
+// part the rounding of what the parts before it leave: 24 bits, all that FP32
+// holds, and every product with a BF16 weight is exact in FP32. (TF32 in two
+// parts, which the tiles below use, keeps 22 bits and takes four instructions
+// where this takes three.)
+__device__ __forceinline__ void mmaBf16(float (&d)[4], const uint32_t (&a)[4], uint2 b) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
+}
+__device__ __forceinline__ uint32_t packBf16(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// the next part of (x, y), which is taken off them
+__device__ __forceinline__ uint32_t nextPart(float& x, float& y) {
+    const uint32_t p = packBf16(x, y);
+    x -= __uint_as_float(p << 16);
+    y -= __uint_as_float(p & 0xFFFF0000u);
+    return p;
+}
+// the three parts of a lane's channels of rows g (r0) and g + 8 (r1), smallest first
+__device__ __forceinline__ void splitRows(float4 r0, float4 r1, uint32_t (&a)[3][4]) {
+#pragma unroll
+    for (int q = 2; q >= 0; q--) {
+        a[q][0] = nextPart(r0.x, r0.y);
+        a[q][1] = nextPart(r1.x, r1.y);
+        a[q][2] = nextPart(r0.z, r0.w);
+        a[q][3] = nextPart(r1.z, r1.w);
+    }
+}
+__device__ __forceinline__ float4 ldv4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ldv4(const bfloat* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xFFFF0000u), __uint_as_float(u.y << 16),
+                       __uint_as_float(u.y & 0xFFFF0000u));
+}
+__device__ __forceinline__ void stv4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void stv4(bfloat* p, float4 v) {
+    *reinterpret_cast<uint2*>(p) = make_uint2(packBf16(v.x, v.y), packBf16(v.z, v.w));
+}
+__device__ __forceinline__ float2 ldv2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 ldv2(const bfloat* p) {
+    const uint32_t u = *reinterpret_cast<const uint32_t*>(p);
+    return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
+}
+__device__ __forceinline__ void stv2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
+__device__ __forceinline__ void stv2(bfloat* p, float2 v) { *reinterpret_cast<uint32_t*>(p) = packBf16(v.x, v.y); }
+__device__ __forceinline__ void add4(float4& a, float4 b) {
+    a.x += b.x;
+    a.y += b.y;
+    a.z += b.z;
+    a.w += b.w;
+}
+
+// The weight groups [K][Cout] of the flat vector in fragment order, for the
+// forward product (inner index K) and the input gradient's (inner index Cout).
+constexpr int kMaxGroups = 24;
+struct PackArgs {
+    int n = 0;
+    unsigned int off[kMaxGroups];
+    short K[kMaxGroups], Cout[kMaxGroups];
+};
+__global__ void __launch_bounds__(kThreads) k_pack(PackArgs a, const bfloat* __restrict__ low, bfloat* __restrict__ fwd,
+                                                   bfloat* __restrict__ bwd) {
+    const unsigned int off = a.off[blockIdx.y];
+    const int K = a.K[blockIdx.y], Cout = a.Cout[blockIdx.y];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < K * Cout; i += gridDim.x * blockDim.x) {
+        const int e = i & 3, lane = (i >> 2) & 31, g = lane >> 2, t4 = lane & 3, blk = i >> 7;
+        const int nf = Cout / 8, nbk = K / 8;  // column blocks
+        fwd[off + i] = low[off + (16 * (blk / nf) + 4 * t4 + e) * Cout + (blk % nf) * 8 + g];
+        bwd[off + i] = low[off + ((blk % nbk) * 8 + g) * Cout + 16 * (blk / nbk) + 4 * t4 + e];
+    }
+}
+
+// The packed weights of `cols` columns and `inner` inner indices into shared memory.
+__device__ __forceinline__ void stageWeights(uint2* ws, const bfloat* packed, int inner, int cols) {
+    const uint4* src = reinterpret_cast<const uint4*>(packed);
+    uint4* dst = reinterpret_cast<uint4*>(ws);
+    for (int i = threadIdx.x; i < inner * cols / 8; i += blockDim.x) dst[i] = __ldg(src + i);
+    __syncthreads();
+}
+
+// acc += the slab's three parts times its weights
+template <int NB>
+__device__ __forceinline__ void slabMma(float (&acc)[NB][4], float4 r0, float4 r1, const uint2* w) {
+    uint32_t a[3][4];
+    splitRows(r0, r1, a);
+#pragma unroll
+    for (int nb = 0; nb < NB; nb++) {
+        const uint2 b = w[nb * 32];
+#pragma unroll
+        for (int q = 0; q < 3; q++) mmaBf16(acc[nb], a[q], b);
+    }
+}
+
+// Sum over a list's rows of the lane's four channels. The first eight entries
+// are in registers (k), further ones are read again for every slab.
+template <class TA>
+__device__ __forceinline__ float4 listSum(const TA* x, int C, const int (&k)[8], int len, const int32_t* more) {
+    float4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (u < len) v[u] = ldv4(x + (size_t)k[u] * C);
+    }
+    add4(v[0], v[1]);
+    add4(v[2], v[3]);
+    add4(v[0], v[2]);
+    if (len > 4) {
+        add4(v[4], v[5]);
+        add4(v[6], v[7]);
+        add4(v[4], v[6]);
+        add4(v[0], v[4]);
+    }
+    for (int u = 8; u < len; u++) add4(v[0], ldv4(x + (size_t)__ldg(more + u) * C));
+    return v[0];
+}
+
+constexpr int kMmaThreads = 128;
+
+// What bounds it: the finest level's tiles, by L2 (each row's inputs are read
+// about five times, its own and its neighbours'), the coarse levels' by the
+// latency of one tile. With the tile kernel, an 874k-cell finest layer took
+// 127 us and a 54-row layer 27; here 81 and 19 (cold caches).
+// Y = act(Z W + b [+ add]): 16-row tiles, Cout / (8 NB) warps of a CTA on one
+// tile's column groups. CTAs loop over tiles with the weights kept.
+template <class TA, int NB>
+__global__ void __launch_bounds__(kMmaThreads) k_layer_mma(const Ctl* ctl, int gated, NetLayer L,
+                                                           const bfloat* __restrict__ P,
+                                                           const bfloat* __restrict__ packed) {
+    if (idle(ctl, gated)) return;
+    extern __shared__ __align__(16) uint2 wsm[];
+    const int K = L.K, Cout = L.Cout;
+    stageWeights(wsm, packed + L.wOff, K, Cout);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const int groups = Cout / (8 * NB), perCta = (kMmaThreads / 32) / groups;
+    const int col0 = (warp % groups) * 8 * NB;
+    const uint2* w0 = wsm + (col0 / 8) * 32 + lane;
+    const int slabW = (Cout / 8) * 32;  // weights of one slab
+    const bfloat* bias = P + L.wOff + (size_t)K * Cout;
+    const TA* add = (const TA*)L.add;
+    TA* Y = (TA*)L.Y;
+    TA* Z = col0 == 0 ? (TA*)L.Z : nullptr;
+    const int tiles = (L.N + 15) / 16;
+    for (int tile = blockIdx.x * perCta + warp / groups; tile < tiles; tile += gridDim.x * perCta) {
+        const int r0 = tile * 16 + g, r1 = r0 + 8;
+        const int n0 = min(r0, L.N - 1), n1 = min(r1, L.N - 1);  // a surplus row repeats the last one and stores nothing
+        float acc[NB][4];
+#pragma unroll
+        for (int nb = 0; nb < NB; nb++) {
+            const float2 b = ldv2(bias + col0 + nb * 8 + 2 * t4);
+            acc[nb][0] = acc[nb][2] = b.x;
+            acc[nb][1] = acc[nb][3] = b.y;
+        }
+        int k0 = 0;
+#pragma unroll 1
+        for (int i = 0; i < L.nIn; i++) {
+            const NetIn& I = L.in[i];
+            const int C = I.C;
+            const TA* x = (const TA*)I.x + 4 * t4;
+            const bool mean = I.xf == NX_NBMEAN || I.xf == NX_POOL;
+            int ka[8], kb[8], la = 0, lb = 0;
+            float ia = 1.f, ib = 1.f;
+            const int32_t *ma = nullptr, *mb = nullptr;
+            if (mean) {
+                const int sa = I.s[n0], sb = I.s[n1];
+                la = I.s[n0 + 1] - sa;
+                lb = I.s[n1 + 1] - sb;
+                ia = I.inv[n0];
+                ib = I.inv[n1];
+                ma = I.list + sa;
+                mb = I.list + sb;
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    ka[u] = u < la ? __ldg(ma + u) : 0;
+                    kb[u] = u < lb ? __ldg(mb + u) : 0;
+                }
+            } else {
+                ka[0] = I.xf == NX_UNPOOL ? I.map[n0] : n0;
+                kb[0] = I.xf == NX_UNPOOL ? I.map[n1] : n1;
+            }
+#pragma unroll 2
+            for (int c = 0; c < C; c += 16, k0 += 16, x += 16) {
+                float4 va, vb;
+                if (mean) {
+                    va = listSum(x, C, ka, la, ma);
+                    vb = listSum(x, C, kb, lb, mb);
+                    va.x *= ia; va.y *= ia; va.z *= ia; va.w *= ia;
+                    vb.x *= ib; vb.y *= ib; vb.z *= ib; vb.w *= ib;
+                } else {
+                    va = ldv4(x + (size_t)ka[0] * C);
+                    vb = ldv4(x + (size_t)kb[0] * C);
+                }
+                if (Z) {
+                    if (r0 < L.N) stv4(Z + (size_t)r0 * K + k0 + 4 * t4, va);
+                    if (r1 < L.N) stv4(Z + (size_t)r1 * K + k0 + 4 * t4, vb);
+                }
+                slabMma<NB>(acc, va, vb, w0 + (k0 / 16) * slabW);
+            }
+        }
+#pragma unroll
+        for (int nb = 0; nb < NB; nb++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int n = h ? r1 : r0;
+                if (n >= L.N) continue;
+                const size_t o = (size_t)n * Cout + col0 + nb * 8 + 2 * t4;
+                float2 v = make_float2(acc[nb][2 * h], acc[nb][2 * h + 1]);
+                if (add) {
+                    const float2 d = ldv2(add + o);
+                    v.x += d.x;
+                    v.y += d.y;
+                }
+                if (L.relu) {
+                    v.x = fmaxf(v.x, 0.f);
+                    v.y = fmaxf(v.y, 0.f);
+                }
+                stv2(Y + o, v);
+            }
+    }
+}
+
+// G = gY act'(Y) (written for the weight gradient) and dZ = G W^T, the same way
+// with Cout as the inner index and K columns.
+template <class TA, int NB>
+__global__ void __launch_bounds__(kMmaThreads) k_layer_dz_mma(NetLayer L, const bfloat* __restrict__ packed,
+                                                              float* __restrict__ G, float* __restrict__ dZ) {
+    extern __shared__ __align__(16) uint2 wsm[];
+    const int K = L.K, Cout = L.Cout;
+    stageWeights(wsm, packed + L.wOff, Cout, K);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const int groups = K / (8 * NB), perCta = (kMmaThreads / 32) / groups;
+    const int col0 = (warp % groups) * 8 * NB;
+    const uint2* w0 = wsm + (col0 / 8) * 32 + lane;
+    const int slabW = (K / 8) * 32;
+    const TA* Y = (const TA*)L.Y;
+    const int tiles = (L.N + 15) / 16;
+    auto masked = [&](int n, int c) {
+        const size_t o = (size_t)n * Cout + c;
+        float4 v = ldv4(L.gY + o);
+        if (L.relu) {
+            const float4 y = ldv4(Y + o);
+            if (y.x <= 0.f) v.x = 0.f;
+            if (y.y <= 0.f) v.y = 0.f;
+            if (y.z <= 0.f) v.z = 0.f;
+            if (y.w <= 0.f) v.w = 0.f;
+        }
+        return v;
+    };
+    for (int tile = blockIdx.x * perCta + warp / groups; tile < tiles; tile += gridDim.x * perCta) {
+        const int r0 = tile * 16 + g, r1 = r0 + 8;
+        const int n0 = min(r0, L.N - 1), n1 = min(r1, L.N - 1);
+        float acc[NB][4];
+#pragma unroll
+        for (int nb = 0; nb < NB; nb++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[nb][e] = 0.f;
+#pragma unroll 2
+        for (int c = 0; c < Cout; c += 16) {
+            const float4 va = masked(n0, c + 4 * t4), vb = masked(n1, c + 4 * t4);
+            if (col0 == 0) {
+                if (r0 < L.N) stv4(G + (size_t)r0 * Cout + c + 4 * t4, va);
+                if (r1 < L.N) stv4(G + (size_t)r1 * Cout + c + 4 * t4, vb);
+            }
+            slabMma<NB>(acc, va, vb, w0 + (c / 16) * slabW);
+        }
+#pragma unroll
+        for (int nb = 0; nb < NB; nb++) {
+            const int o = col0 + nb * 8 + 2 * t4;
+            if (r0 < L.N) stv2(dZ + (size_t)r0 * K + o, make_float2(acc[nb][0], acc[nb][1]));
+            if (r1 < L.N) stv2(dZ + (size_t)r1 * K + o, make_float2(acc[nb][2], acc[nb][3]));
+        }
+    }
+}
+
+// The input layer (two features per row), four lanes a row.
+template <class TA>
+__global__ void __launch_bounds__(kThreads) k_layer_in(const Ctl* ctl, int gated, NetLayer L,
+                                                       const bfloat* __restrict__ P) {
+    if (idle(ctl, gated)) return;
+    const int per = L.Cout / 4;
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t n = i / per;
+    const int o = (int)(i % per) * 4;
+    if (n >= (size_t)L.N) return;
+    const bfloat* W = P + L.wOff;
+    const float2 z = ldv2((const TA*)L.in[0].x + 2 * n);
+    const float4 w0 = ldv4(W + o), w1 = ldv4(W + L.Cout + o), b = ldv4(W + 2 * L.Cout + o);
+    float4 v = make_float4(fmaf(z.y, w1.x, fmaf(z.x, w0.x, b.x)), fmaf(z.y, w1.y, fmaf(z.x, w0.y, b.y)),
+                           fmaf(z.y, w1.z, fmaf(z.x, w0.z, b.z)), fmaf(z.y, w1.w, fmaf(z.x, w0.w, b.w)));
+    if (L.relu) v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+    stv4((TA*)L.Y + n * L.Cout + o, v);
+}
+
+// The output layer (16 channels to one value), four lanes a row.
+template <class TA>
+__global__ void __launch_bounds__(kThreads) k_layer_out(const Ctl* ctl, int gated, NetLayer L,
+                                                        const bfloat* __restrict__ P) {
+    if (idle(ctl, gated)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = i >> 2, t4 = i & 3;
+    const int m = min(n, L.N - 1);
+    const float4 z = ldv4((const TA*)L.in[0].x + (size_t)m * 16 + 4 * t4), w = ldv4(P + L.wOff + 4 * t4);
+    float v = fmaf(z.w, w.w, fmaf(z.z, w.z, fmaf(z.y, w.y, z.x * w.x)));
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+    if (t4 == 0 && n < L.N) stv((TA*)L.Y, n, v + ldv(P, L.wOff + 16));
+}
+
+// Its input gradient straight into the source's: gX[n][k] += g[n] w[k].
+__global__ void __launch_bounds__(kThreads) k_adj_out(NetLayer L, const bfloat* __restrict__ P, float* __restrict__ gX) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = i >> 2, t4 = i & 3;
+    if (n >= L.N) return;
+    const float g = L.gY[n];
+    const float4 w = ldv4(P + L.wOff + 4 * t4);
+    float* p = gX + (size_t)n * 16 + 4 * t4;
+    float4 v = ldv4(p);
+    add4(v, make_float4(g * w.x, g * w.y, g * w.z, g * w.w));
+    stv4(p, v);
+}
+
+// G = gY act'(Y) alone (the input layer has no input gradient)
+template <class TA>
+__global__ void __launch_bounds__(kThreads) k_mask(size_t n4, const float* __restrict__ gY, const TA* __restrict__ Y,
+                                                   float* __restrict__ G) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n4) return;
+    float4 v = ldv4(gY + 4 * i);
+    const float4 y = ldv4(Y + 4 * i);
+    if (y.x <= 0.f) v.x = 0.f;
+    if (y.y <= 0.f) v.y = 0.f;
+    if (y.z <= 0.f) v.z = 0.f;
+    if (y.w <= 0.f) v.w = 0.f;
+    stv4(G + 4 * i, v);
+}
+
 // e = sigma * y
 template <class TA>
 __global__ void __launch_bounds__(kThreads) k_scale_out(const Ctl* ctl, int gated, int N, const TA* y, const double* scal,
@@ -580,7 +934,8 @@ __global__ void __launch_bounds__(kThreads) k_layer_dz(NetLayer L, const TW* __r
 }
 
 // partial[split][K*Cout + Cout] = (Z^T G, sum G) over the split's rows.
-// Block: a 32 x 32 tile of (k, o); 256 threads, 4 k per thread.
+// Block: a 32 x 32 tile of (k, o), 64 rows at a time; the next rows' values are
+// loaded into registers while the current ones are multiplied.
 template <class TA>
 __global__ void __launch_bounds__(kThreads) k_wgrad(int N, int K, int Cout, int tilesO, int rowsPerSplit,
                                                     const TA* __restrict__ Z, const float* __restrict__ G,
@@ -598,15 +953,26 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(int N, int K, int Cout, int 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
     const int mb = warp >> 2, nb = warp & 3;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    float bacc = 0.f;
+    float bacc = 0.f;  // this warp's rows of column o0 + lane
+    float zr[8], gr[8];
+    auto load = [&](int rc) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int n = rc + warp + 8 * u;
+            zr[u] = (n < r1 && k0 + lane < K) ? ldv(Z, (size_t)n * K + k0 + lane) : 0.f;
+            gr[u] = (n < r1 && o0 + lane < Cout) ? G[(size_t)n * Cout + o0 + lane] : 0.f;
+        }
+    };
+    load(r0);
     for (int rc = r0; rc < r1; rc += 64) {
-        for (int i = threadIdx.x; i < 64 * 32; i += kThreads) {
-            const int rr = i >> 5, cc = i & 31;
-            const int n = rc + rr;
-            zs[rr][cc] = (n < r1 && k0 + cc < K) ? ldv(Z, (size_t)n * K + k0 + cc) : 0.f;
-            gs[rr][cc] = (n < r1 && o0 + cc < Cout) ? G[(size_t)n * Cout + o0 + cc] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            zs[warp + 8 * u][lane] = zr[u];
+            gs[warp + 8 * u][lane] = gr[u];
+            bacc += gr[u];
         }
         __syncthreads();
+        if (rc + 64 < r1) load(rc + 64);
 #pragma unroll 2
         for (int kk = 0; kk < 64; kk += 8) {
             const float a[4] = {zs[kk + t4][mb * 16 + g], zs[kk + t4][mb * 16 + g + 8], zs[kk + t4 + 4][mb * 16 + g],
@@ -629,8 +995,6 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(int N, int K, int Cout, int 
             mmaTf32(acc, ahi, blo);
             mmaTf32(acc, ahi, bhi);
         }
-        if (warp == 0)
-            for (int rr = 0; rr < 64; rr++) bacc += gs[rr][lane];
         __syncthreads();
     }
     const size_t stride = (size_t)K * Cout + Cout;
@@ -641,64 +1005,107 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(int N, int K, int Cout, int 
         const int o = o0 + nb * 8 + 2 * t4 + (e & 1);
         if (k < K && o < Cout) out[(size_t)k * Cout + o] = acc[e];
     }
-    if (tk == 0 && warp == 0 && o0 + lane < Cout) out[(size_t)K * Cout + o0 + lane] = bacc;
+    if (tk != 0) return;
+    zs[warp][lane] = bacc;
+    __syncthreads();
+    if (warp == 0 && o0 + lane < Cout) {
+        for (int w = 1; w < kThreads / 32; w++) bacc += zs[w][lane];
+        out[(size_t)K * Cout + o0 + lane] = bacc;
+    }
 }
 
+// grad += the sum of the splits: 32 entries a block, eight threads an entry
 __global__ void __launch_bounds__(kThreads) k_wgrad_reduce(int entries, int splits, const float* __restrict__ partial,
                                                            float* __restrict__ grad) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= entries) return;
+    __shared__ float sh[8][32];
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int e = blockIdx.x * 32 + lane;
     float s = 0.f;
-    for (int i = 0; i < splits; i++) s += partial[(size_t)i * entries + e];
-    grad[e] += s;
+    if (e < entries) {
+#pragma unroll 8
+        for (int i = part; i < splits; i += 8) s += partial[(size_t)i * entries + e];
+    }
+    sh[part][lane] = s;
+    __syncthreads();
+    if (part == 0 && e < entries) {
+        for (int w = 1; w < 8; w++) s += sh[w][lane];
+        grad[e] += s;
+    }
 }
 
-// adjoints: accumulate segment [off, off + C) of dZ (row stride K) into gX
+// adjoints: accumulate segment [off, off + C) of dZ (row stride K) into gX,
+// four channels a thread (every C, K and off is a multiple of four)
+__device__ __forceinline__ void accumulate4(float* p, float4 v) {
+    float4 x = ldv4(p);
+    add4(x, v);
+    stv4(p, x);
+}
+__device__ __forceinline__ float4 scaled(float4 v, float w) { return make_float4(v.x * w, v.y * w, v.z * w, v.w * w); }
+
 __global__ void __launch_bounds__(kThreads) k_adj_id(int N, int C, int off, int K, const float* __restrict__ dZ,
                                                      float* __restrict__ gX) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)N * C) return;
-    const size_t n = i / C, c = i % C;
-    gX[i] += dZ[n * K + off + c];
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)C / 4;
+    if (i >= (size_t)N * per) return;
+    accumulate4(gX + 4 * i, ldv4(dZ + (i / per) * K + off + 4 * (i % per)));
 }
 
-// neighbour mean transposed: gX[k] += sum_{n in nb(k)} invDeg[n] dZ[n]
-__global__ void __launch_bounds__(kThreads) k_adj_nbmean(int N, int C, int off, int K, const int32_t* __restrict__ s,
-                                                         const int32_t* __restrict__ list,
-                                                         const float* __restrict__ inv, const float* __restrict__ dZ,
-                                                         float* __restrict__ gX) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)N * C) return;
-    const int k = (int)(i / C), c = (int)(i % C);
-    float acc = 0.f;
-    for (int q = s[k]; q < s[k + 1]; q++) {
-        const int n = list[q];
-        acc = fmaf(inv[n], dZ[(size_t)n * K + off + c], acc);
+// the message-passing layer's two inputs in one pass: the identity, then the
+// neighbour mean transposed, gX[k] += dZ[k] + sum_{n in nb(k)} invDeg[n] dZ[n]
+__global__ void __launch_bounds__(kThreads) k_adj_mp(int N, int C, int K, const int32_t* __restrict__ s,
+                                                     const int32_t* __restrict__ list, const float* __restrict__ inv,
+                                                     const float* __restrict__ dZ, float* __restrict__ gX) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)C / 4;
+    if (i >= (size_t)N * per) return;
+    const int k = (int)(i / per), c = (int)(i % per) * 4;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int q1 = s[k + 1];
+    for (int q = s[k]; q < q1; q += 4) {
+        int n[4];
+        float w[4];
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) n[u] = list[min(q + u, q1 - 1)];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            w[u] = inv[n[u]];
+            v[u] = ldv4(dZ + (size_t)n[u] * K + C + c);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (q + u < q1) {
+                acc.x = fmaf(w[u], v[u].x, acc.x);
+                acc.y = fmaf(w[u], v[u].y, acc.y);
+                acc.z = fmaf(w[u], v[u].z, acc.z);
+                acc.w = fmaf(w[u], v[u].w, acc.w);
+            }
     }
-    gX[i] += acc;
+    float* p = gX + (size_t)k * C + c;
+    float4 x = ldv4(p);
+    add4(x, ldv4(dZ + (size_t)k * K + c));
+    add4(x, acc);
+    stv4(p, x);
 }
 
 // pool transposed: gX[m] += invCnt[c] dZ[c], c = c2c[m] (m over the fine rows)
 __global__ void __launch_bounds__(kThreads) k_adj_pool(int Nf, int C, int off, int K, const int32_t* __restrict__ c2c,
                                                        const float* __restrict__ invCnt, const float* __restrict__ dZ,
                                                        float* __restrict__ gX) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)Nf * C) return;
-    const int m = (int)(i / C), c = (int)(i % C);
-    const int cc = c2c[m];
-    gX[i] += invCnt[cc] * dZ[(size_t)cc * K + off + c];
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)C / 4;
+    if (i >= (size_t)Nf * per) return;
+    const int cc = c2c[i / per];
+    accumulate4(gX + 4 * i, scaled(ldv4(dZ + (size_t)cc * K + off + 4 * (i % per)), invCnt[cc]));
 }
 
 // unpool transposed: gX[c] += sum_{m in members(c)} dZ[m] (c over the coarse rows)
 __global__ void __launch_bounds__(kThreads) k_adj_unpool(int Nc, int C, int off, int K, const int32_t* __restrict__ ms,
                                                          const int32_t* __restrict__ ml, const float* __restrict__ dZ,
                                                          float* __restrict__ gX) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)Nc * C) return;
-    const int c = (int)(i / C), cc = (int)(i % C);
-    float acc = 0.f;
-    for (int q = ms[c]; q < ms[c + 1]; q++) acc += dZ[(size_t)ml[q] * K + off + cc];
-    gX[i] += acc;
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)C / 4;
+    if (i >= (size_t)Nc * per) return;
+    const int c = (int)(i / per);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = ms[c]; q < ms[c + 1]; q++) add4(acc, ldv4(dZ + (size_t)ml[q] * K + off + 4 * (i % per)));
+    accumulate4(gX + 4 * i, acc);
 }
 
 // ---------------- optimiser ----------------
@@ -814,6 +1221,66 @@ inline bool tileable(const NetLayer& L) {
     return true;
 }
 
+// The fragment kernels take layers whose inputs and outputs come in whole
+// 16-channel slabs of at most 256 and 128 channels: all but the first and the
+// last layer.
+inline bool slabs(const NetLayer& L) {
+    const auto pow2 = [](int c, int most) { return c >= 16 && c <= most && (c & (c - 1)) == 0; };
+    return pow2(L.K, 256) && pow2(L.Cout, 128);
+}
+// Column blocks of eight a warp: up to eight, so a tile's gather is done by as
+// few warps as the registers allow (four on the coarse levels, for more warps a
+// tile, measured no faster: 1.99 against 1.99 ms a prediction on 874k cells,
+// and 2.08 with four on every level).
+inline int mmaBlocks(int cols) { return std::min(cols / 8, 8); }
+
+// One wave of CTAs that loop over the tiles: as many as shared memory (192 KB
+// of weights an SM) and 48 warps an SM allow.
+inline int mmaCtas(const NetLayer& L, int tilesPerCta, size_t smem) {
+    const int perSm = (int)std::min<size_t>(48 * 32 / kMmaThreads, 192 * 1024 / smem);
+    return std::min((L.N + 16 * tilesPerCta - 1) / (16 * tilesPerCta), 148 * perSm);
+}
+
+template <class TA, int NB>
+void launchMmaNB(const Ctl* ctl, int gated, const NetLayer& L, const bfloat* P, const bfloat* packed, cudaStream_t s) {
+    const size_t smem = (size_t)L.K * L.Cout * sizeof(bfloat);
+    allowSmem(k_layer_mma<TA, NB>, smem);
+    const int perCta = (kMmaThreads / 32) / (L.Cout / (8 * NB));
+    k_layer_mma<TA, NB><<<mmaCtas(L, perCta, smem), kMmaThreads, smem, s>>>(ctl, gated, L, P, packed);
+}
+template <class TA>
+void launchMma(const Ctl* ctl, int gated, const NetLayer& L, const bfloat* P, const bfloat* packed, cudaStream_t s) {
+    switch (mmaBlocks(L.Cout)) {
+        case 2: launchMmaNB<TA, 2>(ctl, gated, L, P, packed, s); return;
+        case 4: launchMmaNB<TA, 4>(ctl, gated, L, P, packed, s); return;
+        default: launchMmaNB<TA, 8>(ctl, gated, L, P, packed, s); return;
+    }
+}
+template <class TA, int NB>
+void launchDzMmaNB(const NetLayer& L, const bfloat* packed, float* G, float* dZ, cudaStream_t s) {
+    const size_t smem = (size_t)L.K * L.Cout * sizeof(bfloat);
+    allowSmem(k_layer_dz_mma<TA, NB>, smem);
+    const int perCta = (kMmaThreads / 32) / (L.K / (8 * NB));
+    k_layer_dz_mma<TA, NB><<<mmaCtas(L, perCta, smem), kMmaThreads, smem, s>>>(L, packed, G, dZ);
+}
+template <class TA>
+void launchDzMma(const NetLayer& L, const bfloat* packed, float* G, float* dZ, cudaStream_t s) {
+    switch (mmaBlocks(L.K)) {
+        case 2: launchDzMmaNB<TA, 2>(L, packed, G, dZ, s); return;
+        case 4: launchDzMmaNB<TA, 4>(L, packed, G, dZ, s); return;
+        default: launchDzMmaNB<TA, 8>(L, packed, G, dZ, s); return;
+    }
+}
+
+// A layer with BF16 weights.
+template <class TA>
+void launchLayerLow(const Ctl* ctl, int gated, const NetLayer& L, const bfloat* P, const bfloat* packed,
+                    cudaStream_t s) {
+    if (slabs(L)) launchMma<TA>(ctl, gated, L, P, packed, s);
+    else if (L.K == 2) k_layer_in<TA><<<blocksFor((size_t)L.N * L.Cout / 4), kThreads, 0, s>>>(ctl, gated, L, P);
+    else k_layer_out<TA><<<blocksFor((size_t)L.N * 4), kThreads, 0, s>>>(ctl, gated, L, P);
+}
+
 template <class TA, class TW>
 void launchLayerFwd(const Ctl* ctl, int gated, const NetLayer& L, const void* P, cudaStream_t s) {
     switch (tileable(L) ? L.Cout : 0) {
@@ -863,7 +1330,12 @@ T* devUpload(std::vector<void*>& list, const std::vector<T>& h) {
     return d;
 }
 
-inline int wgradSplits(int rows) { return std::min(512, std::max(1, (rows + 2047) / 2048)); }
+// Splits of a layer's rows for its weight gradient: enough blocks (with its
+// 32 x 32 tiles) for eight on each of 148 SMs, and at least 128 rows in each.
+inline int wgradSplits(const NetLayer& L) {
+    const int tiles = ((L.K + 31) / 32) * ((L.Cout + 31) / 32);
+    return std::max(1, std::min((L.N + 127) / 128, (1184 + tiles - 1) / tiles));
+}
 
 }  // namespace
 
@@ -962,6 +1434,15 @@ void LearnedNet::buildLayers() {
     auto act = [&](size_t n) { return (void*)devAlloc<unsigned char>(allocs_, n * tsz); };
     auto grd = [&](size_t n) { return devAlloc<float>(allocs_, n); };
     const int L = L_;
+    // the activations' gradients in one block, zeroed together before a backward pass
+    gradActs_ = 0;
+    for (int l = 0; l < L; l++) gradActs_ += 4 * (size_t)g_[(size_t)l].N * C_[(size_t)l];
+    gActs_ = grd(gradActs_);
+    size_t gUsed = 0;
+    auto actGrd = [&](size_t n) {
+        gUsed += n;
+        return gActs_ + gUsed - n;
+    };
     std::vector<void*> H((size_t)L), E((size_t)L), S((size_t)L), D((size_t)L);
     std::vector<float*> gH((size_t)L), gE((size_t)L), gS((size_t)L), gD((size_t)L);
     for (int l = 0; l < L; l++) {
@@ -970,10 +1451,10 @@ void LearnedNet::buildLayers() {
         E[(size_t)l] = act(n);
         S[(size_t)l] = act(n);
         D[(size_t)l] = act(n);
-        gH[(size_t)l] = grd(n);
-        gE[(size_t)l] = grd(n);
-        gS[(size_t)l] = grd(n);
-        gD[(size_t)l] = grd(n);
+        gH[(size_t)l] = actGrd(n);
+        gE[(size_t)l] = actGrd(n);
+        gS[(size_t)l] = actGrd(n);
+        gD[(size_t)l] = actGrd(n);
     }
     feat_ = act((size_t)N0_ * 2);
     out_ = act((size_t)N0_);
@@ -1102,6 +1583,10 @@ void LearnedNet::buildLayers() {
     nParams_ = total;
     params_ = devAlloc<float>(allocs_, nParams_);
     paramsLow_ = wBf16_ ? (void*)devAlloc<bfloat>(allocs_, nParams_) : (void*)params_;
+    if (wBf16_) {
+        packF_ = devAlloc<bfloat>(allocs_, nParams_);
+        packB_ = devAlloc<bfloat>(allocs_, nParams_);
+    }
     grad_ = devAlloc<float>(allocs_, nParams_);
     adamM_ = devAlloc<float>(allocs_, nParams_);
     adamV_ = devAlloc<float>(allocs_, nParams_);
@@ -1111,7 +1596,7 @@ void LearnedNet::buildLayers() {
         Ly.Z = act((size_t)Ly.N * Ly.K);
         maxG = std::max(maxG, (size_t)Ly.N * Ly.Cout);
         maxZ = std::max(maxZ, (size_t)Ly.N * Ly.K);
-        maxPart = std::max(maxPart, (size_t)wgradSplits(Ly.N) * ((size_t)Ly.K * Ly.Cout + Ly.Cout));
+        maxPart = std::max(maxPart, (size_t)wgradSplits(Ly) * ((size_t)Ly.K * Ly.Cout + Ly.Cout));
     }
     gpre_ = grd(maxG);
     dZ_ = grd(maxZ);
@@ -1125,14 +1610,33 @@ void LearnedNet::buildLayers() {
 void LearnedNet::syncLowPrecision(cudaStream_t s) {
     if (!wBf16_) return;
     k_to_low<bfloat><<<blocksFor(nParams_), kThreads, 0, s>>>(nParams_, params_, (bfloat*)paramsLow_);
+    packWeights(s);
     NCK(cudaGetLastError());
+}
+
+// The weights in fragment order, after every change of them.
+void LearnedNet::packWeights(cudaStream_t s) {
+    PackArgs a;
+    a.n = 0;
+    for (const NetLayer& L : layers_) {
+        if (!slabs(L)) continue;
+        bool seen = false;
+        for (int i = 0; i < a.n; i++) seen |= a.off[i] == (unsigned)L.wOff;
+        if (seen) continue;
+        if (a.n == kMaxGroups) throw std::runtime_error("too many weight groups");
+        a.off[a.n] = (unsigned)L.wOff;
+        a.K[a.n] = (short)L.K;
+        a.Cout[a.n] = (short)L.Cout;
+        a.n++;
+    }
+    if (a.n) k_pack<<<dim3(16, a.n), kThreads, 0, s>>>(a, (const bfloat*)paramsLow_, (bfloat*)packF_, (bfloat*)packB_);
 }
 
 void LearnedNet::forward(const Ctl* ctl, int gated, bool keepZ, cudaStream_t s) {
     for (NetLayer L : layers_) {
         if (!keepZ) L.Z = nullptr;
-        if (actBf16_) launchLayerFwd<bfloat, bfloat>(ctl, gated, L, paramsLow_, s);
-        else if (wBf16_) launchLayerFwd<float, bfloat>(ctl, gated, L, paramsLow_, s);
+        if (actBf16_) launchLayerLow<bfloat>(ctl, gated, L, (const bfloat*)paramsLow_, (const bfloat*)packF_, s);
+        else if (wBf16_) launchLayerLow<float>(ctl, gated, L, (const bfloat*)paramsLow_, (const bfloat*)packF_, s);
         else launchLayerFwd<float, float>(ctl, gated, L, paramsLow_, s);
     }
 }
@@ -1156,36 +1660,51 @@ void LearnedNet::backward(cudaStream_t s) {
     for (int i = (int)layers_.size() - 1; i >= 0; i--) {
         const NetLayer& L = layers_[(size_t)i];
         const bool needDz = L.gIn[0] != nullptr;
-        if (actBf16_) launchLayerDz<bfloat, bfloat>(L, paramsLow_, gpre_, needDz ? dZ_ : nullptr, s);
-        else if (wBf16_) launchLayerDz<float, bfloat>(L, paramsLow_, gpre_, needDz ? dZ_ : nullptr, s);
-        else launchLayerDz<float, float>(L, paramsLow_, gpre_, needDz ? dZ_ : nullptr, s);
-        // dW, db
-        const int splits = wgradSplits(L.N);
+        const float* G = gpre_;
+        const bool direct = wBf16_ && needDz && !slabs(L);  // the output layer: its input gradient in one pass
+        if (!wBf16_) {
+            launchLayerDz<float, float>(L, paramsLow_, gpre_, needDz ? dZ_ : nullptr, s);
+        } else if (direct) {
+            G = L.gY;
+            k_adj_out<<<blocksFor((size_t)L.N * 4), kThreads, 0, s>>>(L, (const bfloat*)paramsLow_, L.gIn[0]);
+        } else if (!needDz) {
+            const size_t n4 = (size_t)L.N * L.Cout / 4;
+            if (actBf16_) k_mask<bfloat><<<blocksFor(n4), kThreads, 0, s>>>(n4, L.gY, (const bfloat*)L.Y, gpre_);
+            else k_mask<float><<<blocksFor(n4), kThreads, 0, s>>>(n4, L.gY, (const float*)L.Y, gpre_);
+        } else if (actBf16_) {
+            launchDzMma<bfloat>(L, (const bfloat*)packB_, gpre_, dZ_, s);
+        } else {
+            launchDzMma<float>(L, (const bfloat*)packB_, gpre_, dZ_, s);
+        }
+        // dW, db; a layer with one untransformed input has that as its Z
+        const void* Z = wBf16_ && L.nIn == 1 && L.in[0].xf == NX_ID ? L.in[0].x : L.Z;
+        const int splits = wgradSplits(L);
         const int rowsPerSplit = (L.N + splits - 1) / splits;
         const int tilesK = (L.K + 31) / 32, tilesO = (L.Cout + 31) / 32;
         const dim3 grid((unsigned)(tilesK * tilesO), (unsigned)splits);
         if (actBf16_)
-            k_wgrad<bfloat><<<grid, kThreads, 0, s>>>(L.N, L.K, L.Cout, tilesO, rowsPerSplit, (const bfloat*)L.Z, gpre_,
+            k_wgrad<bfloat><<<grid, kThreads, 0, s>>>(L.N, L.K, L.Cout, tilesO, rowsPerSplit, (const bfloat*)Z, G,
                                                       wgPartial_);
         else
-            k_wgrad<float><<<grid, kThreads, 0, s>>>(L.N, L.K, L.Cout, tilesO, rowsPerSplit, (const float*)L.Z, gpre_,
+            k_wgrad<float><<<grid, kThreads, 0, s>>>(L.N, L.K, L.Cout, tilesO, rowsPerSplit, (const float*)Z, G,
                                                      wgPartial_);
         const int entries = L.K * L.Cout + L.Cout;
-        k_wgrad_reduce<<<blocksFor(entries), kThreads, 0, s>>>(entries, splits, wgPartial_, grad_ + L.wOff);
+        k_wgrad_reduce<<<blocksFor(entries, 32), kThreads, 0, s>>>(entries, splits, wgPartial_, grad_ + L.wOff);
         // adjoints of the inputs
         int off = 0;
-        for (int q = 0; q < L.nIn; q++) {
+        if (L.nIn == 2) {  // message passing: both inputs are the same tensor
+            const NetIn& I = L.in[1];
+            k_adj_mp<<<blocksFor((size_t)L.N * I.C / 4), kThreads, 0, s>>>(L.N, I.C, L.K, I.s, I.list, I.inv, dZ_,
+                                                                         L.gIn[1]);
+        }
+        for (int q = 0; q < L.nIn && L.nIn == 1 && !direct; q++) {
             const NetIn& I = L.in[q];
             float* gX = L.gIn[q];
             if (gX) {
-                const size_t n = (size_t)I.srcRows * I.C;
+                const size_t n = (size_t)I.srcRows * I.C / 4;
                 switch (I.xf) {
                     case NX_ID:
                         k_adj_id<<<blocksFor(n), kThreads, 0, s>>>(I.srcRows, I.C, off, L.K, dZ_, gX);
-                        break;
-                    case NX_NBMEAN:
-                        k_adj_nbmean<<<blocksFor(n), kThreads, 0, s>>>(I.srcRows, I.C, off, L.K, I.s, I.list, I.inv,
-                                                                      dZ_, gX);
                         break;
                     case NX_POOL:
                         k_adj_pool<<<blocksFor(n), kThreads, 0, s>>>(I.srcRows, I.C, off, L.K, I.map, I.inv, dZ_, gX);
@@ -1198,7 +1717,7 @@ void LearnedNet::backward(cudaStream_t s) {
             off += I.C;
         }
         if (L.gAdd) {
-            const size_t n = (size_t)L.N * L.Cout;
+            const size_t n = (size_t)L.N * L.Cout / 4;
             k_adj_id<<<blocksFor(n), kThreads, 0, s>>>(L.N, L.Cout, 0, L.Cout, gpre_, L.gAdd);
         }
     }
@@ -1223,8 +1742,7 @@ void LearnedNet::lossAndGrad(const Sample& smp, float* lossOut, cudaStream_t s) 
                                                     smp.target, Ay_, red_, counter_, scal_);
     k_loss_grad<<<nb0, kThreads, 0, s>>>(N0_, smp.b, Ay_, scal_, gOut_, lossOut);
     // zero every activation gradient except the output's, and the parameter gradient
-    for (const NetLayer& L : layers_)
-        if (L.gY != gOut_) NCK(cudaMemsetAsync(L.gY, 0, (size_t)L.N * L.Cout * sizeof(float), s));
+    NCK(cudaMemsetAsync(gActs_, 0, gradActs_ * sizeof(float), s));
     NCK(cudaMemsetAsync(grad_, 0, nParams_ * sizeof(float), s));
     backward(s);
 }
@@ -1253,6 +1771,7 @@ void LearnedNet::trainStep(const Sample& smp, float lr, int t, float* lossOut, c
     if (wBf16_)
         k_adam<bfloat><<<blocksFor(nParams_), kThreads, 0, s>>>(nParams_, params_, grad_, adamM_, adamV_,
                                                                 (bfloat*)paramsLow_, lr, b1, b2, 1e-8f, c1, c2);
+    if (wBf16_) packWeights(s);
     else
         k_adam<float><<<blocksFor(nParams_), kThreads, 0, s>>>(nParams_, params_, grad_, adamM_, adamV_, params_, lr,
                                                                b1, b2, 1e-8f, c1, c2);

@@ -141,6 +141,7 @@ public:
 private:
     void release();
     void buildLayers();
+    void packWeights(cudaStream_t s);
     void forward(const Ctl* ctl, int gated, bool keepZ, cudaStream_t s);
     void backward(cudaStream_t s);
 
@@ -153,6 +154,8 @@ private:
     // parameters
     float* params_ = nullptr;
     void* paramsLow_ = nullptr;  // BF16 copies (or the FP32 masters in FP32 mode)
+    void* packF_ = nullptr;  // BF16 weights in fragment order, for the forward and the input gradient's products
+    void* packB_ = nullptr;
     float* grad_ = nullptr;
     float* adamM_ = nullptr;
     float* adamV_ = nullptr;
@@ -161,6 +164,8 @@ private:
     void* feat_ = nullptr;  // [N0][2]
     void* out_ = nullptr;   // [N0]
     float* gOut_ = nullptr;
+    float* gActs_ = nullptr;  // gradients of the layers' outputs
+    size_t gradActs_ = 0;
     float* gpre_ = nullptr;
     float* dZ_ = nullptr;
     const int32_t* nb0_ = nullptr;  // finest level ELL neighbours [W0][N0]

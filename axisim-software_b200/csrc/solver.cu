@@ -349,8 +349,7 @@ public:
         requireNet();
         if (idx < 0 || idx >= learnedSampleCount()) throw StatusError(AXISIM_E_ARG, "sample index out of range");
         if (grad && n != (int64_t)net_.numParams()) throw StatusError(AXISIM_E_ARG, "parameter count mismatch");
-        Arena tmp;
-        float* loss = tmp.alloc<float>(1);
+        float* loss = netScratch() + 4 * (size_t)N_;
         net_.lossAndGrad(sample(idx), loss, stream_);
         CK(cudaStreamSynchronize(stream_));
         float h = 0.f;
@@ -383,8 +382,7 @@ public:
     void learnedPredict(const float* r, const float* ac, const float* d, float* out) {
         requireNet();
         if (!r || !ac || !d || !out) throw StatusError(AXISIM_E_ARG, "array is null");
-        Arena tmp;
-        float* dev = tmp.alloc<float>(4 * (size_t)N_);
+        float* dev = netScratch();
         const float* src[3] = {r, ac, d};
         for (int k = 0; k < 3; k++)
             CK(cudaMemcpy(dev + (size_t)k * N_, src[k], (size_t)N_ * sizeof(float), cudaMemcpyHostToDevice));
@@ -408,6 +406,13 @@ public:
         if (fallbacks) *fallbacks = h.fallbacks;
         if (scoreNet) *scoreNet = h.logRhoNet;
         if (scoreV) *scoreV = h.logRhoV;
+    }
+
+    // 4 N_ + 1 floats for the network's calls, kept while the handle keeps its
+    // mesh (allocated per call, they cost more than the inference itself)
+    float* netScratch() {
+        if (!netScratch_) netScratch_ = netArena_.alloc<float>(4 * (size_t)N_ + 1);
+        return netScratch_;
     }
 
     void ensureNetStats() {
@@ -471,6 +476,7 @@ public:
         fcgR_ = nullptr;
         netArena_.release();
         netStats_ = nullptr;
+        netScratch_ = nullptr;
         nnY_ = nullptr;
         nnAy_ = nullptr;
         resetLearned();
@@ -618,6 +624,7 @@ public:
             fcgR_ = nullptr;
             netArena_.release();
             netStats_ = nullptr;
+            netScratch_ = nullptr;
             nnY_ = nullptr;
             nnAy_ = nullptr;
             resetLearned();
@@ -927,6 +934,7 @@ private:
     // counters of the Krylov steps (V-cycle reduction, learned-step outcomes)
     Arena netArena_;
     NetStats* netStats_ = nullptr;
+    float* netScratch_ = nullptr;
     float* nnY_ = nullptr;    // the network's output in the first Krylov iteration
     double* nnAy_ = nullptr;  // A times it
     // learned preconditioner and its harvested (b, p', A_C, deficit, A_F)
