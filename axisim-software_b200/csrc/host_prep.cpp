@@ -816,13 +816,9 @@ std::vector<int32_t> slotNeighbours(int N, int W, const int32_t* cfs, const int3
     return nb;
 }
 
-SweepTiles buildSweepTiles(int N, int W, const int32_t* nb, const double* cz, const double* cr, int S, int cap,
-                           int tileCells, const int32_t* caseStart, int nCases) {
-    SweepTiles t;
-    t.S = S;
-    t.cap = cap;
-    t.tileStart.assign(1, 0);
-    if (N <= 0 || W < 1 || W > 4 || S < 1 || cap < 1 || cap >= 0xFFFF || tileCells < 1) return t;
+// The cells along a Morton curve of their centres: exact within buckets of more
+// than `refine` cells, by cell id within smaller ones.
+static std::vector<int32_t> curveOrder(int N, const double* cz, const double* cr, int refine) {
     double z0 = cz[0], z1 = cz[0], r0 = cr[0], r1 = cr[0];
     for (int n = 1; n < N; n++) {
         z0 = std::min(z0, cz[n]);
@@ -843,9 +839,8 @@ SweepTiles buildSweepTiles(int N, int W, const int32_t* nb, const double* cz, co
     });
     // cells by key: a counting sort on the top 16 bits (a 256 x 256 grid of
     // the bounding square; per-thread counts, so each bucket keeps ascending
-    // cell order), then buckets of more than half a run by the whole key
-    const int refine = std::max(64, tileCells / 2);
-    std::vector<int32_t> order((size_t)N), tmp((size_t)N);
+    // cell order), then large buckets by the whole key
+    std::vector<int32_t> order((size_t)N);
     {
         const unsigned hw = std::thread::hardware_concurrency();
         const int nt = std::max(1, std::min({(int)(hw ? hw : 1), 16, N / 16384}));
@@ -885,6 +880,18 @@ SweepTiles buildSweepTiles(int N, int W, const int32_t* nb, const double* cz, co
             }
         }, 4096);
     }
+    return order;
+}
+
+SweepTiles buildSweepTiles(int N, int W, const int32_t* nb, const double* cz, const double* cr, int S, int cap,
+                           int tileCells, const int32_t* caseStart, int nCases) {
+    SweepTiles t;
+    t.S = S;
+    t.cap = cap;
+    t.tileStart.assign(1, 0);
+    if (N <= 0 || W < 1 || W > 4 || S < 1 || cap < 1 || cap >= 0xFFFF || tileCells < 1) return t;
+    // buckets of more than half a run are sorted by the whole key
+    std::vector<int32_t> order = curveOrder(N, cz, cr, std::max(64, tileCells / 2)), tmp((size_t)N);
     if (nCases > 1) {  // stable by case: the curve of case 0, then of case 1, ...
         std::vector<int32_t> at((size_t)nCases + 1);
         std::copy(caseStart, caseStart + nCases + 1, at.begin());
@@ -933,6 +940,121 @@ SweepTiles buildSweepTiles(int N, int W, const int32_t* nb, const double* cz, co
         }
     }, 4);
     t.tileStart[nT] = (int32_t)nL;
+    return t;
+}
+
+SweepChunks buildSweepChunks(int N, int W, const int32_t* nb, const double* cz, const double* cr, int chunks,
+                             const int32_t* color, int nColors) {
+    SweepChunks t;
+    if (N <= 0 || W < 1 || W > 4 || chunks < 1 || chunks > 1024 || nColors < 1 || nColors > SweepChunks::kMaxColors)
+        return t;
+    const int per = (N + chunks - 1) / chunks;
+    chunks = (N + per - 1) / per;
+    if (per >= 0x7000) return t;
+    t.cells = chunks > 1 ? curveOrder(N, cz, cr, std::max(32, per / 8)) : std::vector<int32_t>();
+    if (chunks == 1) {
+        t.cells.resize((size_t)N);
+        for (int n = 0; n < N; n++) t.cells[(size_t)n] = n;
+    }
+    t.info.resize((size_t)chunks);
+    std::vector<int16_t> chunkOf((size_t)N);
+    parallelFor(chunks, [&](int c0, int c1) {
+        for (int c = c0; c < c1; c++)
+            for (int p = c * per, e = std::min(N, p + per); p < e; p++) chunkOf[(size_t)t.cells[(size_t)p]] = (int16_t)c;
+    }, 4);
+    // rows of a chunk: by colour, within it those that other chunks read first, then by cell
+    std::vector<int32_t> posOf((size_t)N);  // position of a cell in t.cells
+    std::vector<char> exported((size_t)N);
+    parallelFor(chunks, [&](int c0, int c1) {
+        for (int c = c0; c < c1; c++) {
+            SweepChunks::Info& I = t.info[(size_t)c];
+            I.row0 = c * per;
+            I.rows = std::min(N, I.row0 + per) - I.row0;
+            int32_t* b = t.cells.data() + I.row0;
+            for (int i = 0; i < I.rows; i++) {
+                const int n = b[i];
+                char x = 0;
+                for (int j = 0; j < W; j++) {
+                    const int m = nb[(size_t)j * N + n];
+                    if (m >= 0 && chunkOf[(size_t)m] != c) x = 1;
+                }
+                exported[(size_t)n] = x;
+            }
+            auto rank = [&](int n) { return 2 * (color ? color[n] : 0) + (exported[(size_t)n] ? 0 : 1); };
+            std::sort(b, b + I.rows, [&](int32_t x, int32_t y) {
+                const int rx = rank(x), ry = rank(y);
+                return rx != ry ? rx < ry : x < y;
+            });
+            int at = 0;
+            for (int k = 0; k < nColors; k++) {
+                I.start[k] = at;
+                while (at < I.rows && rank(b[at]) == 2 * k) at++;
+                I.boundary[k] = at;
+                while (at < I.rows && rank(b[at]) == 2 * k + 1) at++;
+            }
+            I.start[nColors] = at;
+            for (int i = 0; i < I.rows; i++) posOf[(size_t)b[i]] = I.row0 + i;
+        }
+    }, 4);
+    // halos, then the rows' local references
+    std::vector<std::vector<int32_t>> halo((size_t)chunks);
+    t.ref.assign(4 * (size_t)N, 0);
+    std::vector<char> ok((size_t)chunks, 1);
+    parallelFor(chunks, [&](int c0, int c1) {
+        for (int c = c0; c < c1; c++) {
+            const SweepChunks::Info& I = t.info[(size_t)c];
+            std::vector<int32_t>& h = halo[(size_t)c];
+            for (int i = 0; i < I.rows; i++)
+                for (int j = 0; j < W; j++) {
+                    const int m = nb[(size_t)j * N + t.cells[(size_t)(I.row0 + i)]];
+                    if (m >= 0 && chunkOf[(size_t)m] != c) h.push_back(posOf[(size_t)m]);
+                }
+            std::sort(h.begin(), h.end());
+            h.erase(std::unique(h.begin(), h.end()), h.end());
+            const int zero = I.rows + (int)h.size();
+            if (zero >= 0x8000) {
+                ok[(size_t)c] = 0;
+                continue;
+            }
+            for (int i = 0; i < I.rows; i++)
+                for (int j = 0; j < 4; j++) {
+                    const int m = j < W ? nb[(size_t)j * N + t.cells[(size_t)(I.row0 + i)]] : -1;
+                    int r = zero;
+                    if (m >= 0)
+                        r = chunkOf[(size_t)m] == c
+                                ? posOf[(size_t)m] - I.row0
+                                : I.rows + (int)(std::lower_bound(h.begin(), h.end(), posOf[(size_t)m]) - h.begin());
+                    t.ref[4 * (size_t)(I.row0 + i) + (size_t)j] = (uint16_t)r;
+                }
+        }
+    }, 4);
+    for (int c = 0; c < chunks; c++) {
+        SweepChunks::Info& I = t.info[(size_t)c];
+        I.halo0 = (int32_t)t.halo.size();
+        I.halos = (int32_t)halo[(size_t)c].size();
+        t.halo.insert(t.halo.end(), halo[(size_t)c].begin(), halo[(size_t)c].end());
+        t.maxRows = std::max(t.maxRows, I.rows);
+        t.maxHalo = std::max(t.maxHalo, I.halos);
+        if (!ok[(size_t)c]) return SweepChunks();
+    }
+    {  // the halos, seen from the rows that fill them
+        std::vector<int32_t> count((size_t)N + 1, 0);
+        for (int p : t.halo) count[(size_t)p + 1]++;
+        for (int p = 0; p < N; p++) count[(size_t)p + 1] += count[(size_t)p];
+        t.push.resize(t.halo.size());
+        std::vector<int32_t> fill(count.begin(), count.end() - 1);
+        for (int c = 0; c < chunks; c++) {
+            const SweepChunks::Info& I = t.info[(size_t)c];
+            for (int h = 0; h < I.halos; h++)
+                t.push[(size_t)fill[(size_t)t.halo[(size_t)(I.halo0 + h)]]++] = (uint32_t)c << 16 | (uint32_t)(I.rows + h);
+        }
+        for (SweepChunks::Info& I : t.info) {
+            I.push0 = count[(size_t)I.row0];
+            I.pushes = count[(size_t)(I.row0 + I.rows)] - I.push0;
+            t.maxPush = std::max(t.maxPush, I.pushes);
+            t.pushAt.insert(t.pushAt.end(), count.begin() + I.row0, count.begin() + I.row0 + I.rows + 1);
+        }
+    }
     return t;
 }
 

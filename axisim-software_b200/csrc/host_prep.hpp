@@ -150,6 +150,30 @@ std::vector<int32_t> slotNeighbours(int nCells, int W, const int32_t* cellFaceSt
 SweepTiles buildSweepTiles(int nCells, int W, const int32_t* nb, const double* cz, const double* cr, int S, int cap,
                            int tileCells, const int32_t* caseStart = nullptr, int nCases = 0);
 
+// The mesh in `chunks` pieces of equal size along a curve of the cell centres,
+// for linear sweeps that stay on the chip (sweep_chunks.cu): a piece's rows by
+// colour, those that other pieces read first, and its halo, the cells of other
+// pieces that its rows refer to. nb is the slot neighbour block [W][N], W <= 4;
+// color (null: one colour) orders Gauss-Seidel sweeps. No pieces when they do
+// not fit 15-bit local references.
+struct SweepChunks {
+    static constexpr int kMaxColors = 8;
+    struct Info {
+        int32_t row0 = 0, rows = 0, halo0 = 0, halos = 0, push0 = 0, pushes = 0;
+        int32_t start[kMaxColors + 1] = {};  // first row of each colour (and the end)
+        int32_t boundary[kMaxColors] = {};   // end of the colour's rows that other pieces read
+    };
+    std::vector<Info> info;
+    std::vector<int32_t> cells;   // rows of all pieces, piece by piece
+    std::vector<int32_t> halo;    // positions in `cells`
+    std::vector<uint16_t> ref;    // four per row: local rows, then halo, then the zero cell of an unused slot
+    std::vector<int32_t> pushAt;  // rows + 1 per piece: a row's run of `push`
+    std::vector<uint32_t> push;   // the halo cells that hold the row: piece << 16 | local cell
+    int maxRows = 0, maxHalo = 0, maxPush = 0;
+};
+SweepChunks buildSweepChunks(int nCells, int W, const int32_t* nb, const double* cz, const double* cr, int chunks,
+                             const int32_t* color, int nColors);
+
 // buildMeshColoring (memory_manger.cpp:334-409): greedy colour per cell.
 int greedyColoring(const GridLevel& g, std::vector<int32_t>& color);
 

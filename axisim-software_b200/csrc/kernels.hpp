@@ -154,6 +154,41 @@ struct ClusterArgsT {
     ClusterStep steps[kMaxClusterSteps];
 };
 
+// All linear sweeps of a system in one launch (sweep_chunks.cu). The host's
+// SweepChunks on the device: one CTA per chunk, the CTAs one cluster.
+constexpr int kSweepClusterChunks = 16;
+constexpr size_t kSweepChunkShared = 220 * 1024;
+struct SweepChunkInfo {
+    int32_t row0, rows, halo0, halos, push0, pushes;
+    int32_t start[9], boundary[8];
+};
+struct SweepChunksDev {
+    int chunks = 0, rowsMax = 0, cellsMax = 0, pushMax = 0;  // cellsMax: rows, halo and zero cell of any chunk
+    const SweepChunkInfo* info = nullptr;
+    const int32_t* cells = nullptr;
+    const int32_t* halo = nullptr;
+    const ushort4* ref = nullptr;
+    const int32_t* pushAt = nullptr;  // rows + 1 entries per chunk, each row's run of `push`
+    const unsigned* push = nullptr;   // chunk << 16 | halo cell there
+};
+// NV systems with one matrix: off-diagonals [W][N], right-hand sides, inverse
+// diagonals, iterates (in place; or, with addTo, addTo += the result).
+template <class T, int NV>
+struct SweepSystem {
+    int N = 0;
+    const T* AF = nullptr;
+    const T* b[NV] = {};
+    const T* inv[NV] = {};
+    T* x[NV] = {};
+    double* addTo[NV] = {};
+};
+bool sweepChunksFit(const SweepChunksDev& d, bool fp32, bool gaussSeidel);
+// `sweeps` Jacobi sweeps, or multicolour Gauss-Seidel sweeps of `colors` colours
+// (0: Jacobi); false when the system does not fit or there are fewer than two sweeps
+template <class T, int NV>
+bool launchSweepChunks(const Ctl* ctl, const SweepChunksDev& d, const SweepSystem<T, NV>& a, int sweeps, int colors,
+                       cudaStream_t s);
+
 // ---- setup ----
 void launchPrecompute(const MeshDev& m, const int32_t* cfs, const int32_t* cfi, double* lsqDZ, double* lsqDR,
                       cudaStream_t s);

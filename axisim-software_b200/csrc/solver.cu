@@ -498,6 +498,9 @@ public:
         copyParallel(hOwner_, pm.faceOwner, (size_t)F);
         copyParallel(hNeighbor_, pm.faceNeighbor, (size_t)F);
         dropSweepTiles();
+        chunkArena_.release();
+        chunks_ = SweepChunksDev();
+        chunkKey_ = 0;
         ph.reset(new PhaseTimer(*this, "mesh_upload"));
         Arena& A = meshArena_;
         // the mesh, its precomputed geometry and the fields below, in one
@@ -1411,6 +1414,68 @@ private:
     }
     double tileLocal_ = 0.0;  // local cells of all tiles (layer 0 and halo)
 
+    // Pieces of the mesh for all sweeps of a solve in one launch: one CTA up to
+    // kSweepCtaCells cells, a cluster of 16 up to kSweepClusterCells; larger
+    // meshes keep a launch per sweep. Whole 20-iteration runs, on chip against a
+    // launch per sweep: 13.7k cells 3.87 / 4.19 ms FP64, 3.60 / 3.78 mixed; 28k
+    // cells 4.36 / 4.53 and 3.96 / 4.10; 53k cells 9.04 / 8.62 (mixed, 40
+    // iterations): 16 SMs become the bound, and the pieces take the host 60 us per
+    // thousand cells, so the line is where it pays within some 50 iterations.
+    static constexpr int kSweepCtaCells = 2048;
+    static constexpr int kSweepClusterCells = 16384;
+    void ensureSweepChunks() {
+        const bool gs = cs_.type == 1, fp32 = precision_ == AXISIM_PREC_MIXED && !gs;
+        const int colors = gs ? colorN_ : 1;
+        const int key = 1 + (gs ? 1 : 0) + (fp32 ? 2 : 0);
+        if (chunkKey_ == key) return;
+        chunkKey_ = key;
+        chunkArena_.release();
+        chunks_ = SweepChunksDev();
+        if (W_ < 3 || W_ > 4 || colors < 1 || colors > SweepChunks::kMaxColors) return;
+        if (N_ > kSweepClusterCells) return;
+        PhaseTimer ph(*this, "sweep_chunks");
+        const std::vector<int32_t> nb =
+            slotNeighbours(N_, W_, hCfs_.data(), hCfi_.data(), hOwner_.data(), hNeighbor_.data());
+        std::vector<double> cz((size_t)N_), cr((size_t)N_);
+        CK(cudaMemcpy(cz.data(), mesh_.ccZ, (size_t)N_ * sizeof(double), cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(cr.data(), mesh_.ccR, (size_t)N_ * sizeof(double), cudaMemcpyDeviceToHost));
+        int want = N_ <= kSweepCtaCells ? 1 : kSweepClusterChunks;
+        for (;;) {
+            SweepChunks t = buildSweepChunks(N_, W_, nb.data(), cz.data(), cr.data(), want, gs ? hColor_.data() : nullptr,
+                                             colors);
+            SweepChunksDev d;
+            d.chunks = (int)t.info.size();
+            d.rowsMax = t.maxRows;
+            d.cellsMax = t.maxRows + t.maxHalo + 1;
+            d.pushMax = t.maxPush;
+            if (d.chunks == want && sweepChunksFit(d, fp32, gs)) {
+                std::vector<SweepChunkInfo> info(t.info.size());
+                for (size_t i = 0; i < info.size(); i++) {
+                    const SweepChunks::Info& f = t.info[i];
+                    SweepChunkInfo& o = info[i];
+                    o.row0 = f.row0; o.rows = f.rows; o.halo0 = f.halo0; o.halos = f.halos;
+                    o.push0 = f.push0; o.pushes = f.pushes;
+                    std::copy(f.start, f.start + 9, o.start);
+                    std::copy(f.boundary, f.boundary + 8, o.boundary);
+                }
+                Arena& A = chunkArena_;
+                d.info = A.upload(info.data(), info.size());
+                d.cells = A.upload(t.cells.data(), t.cells.size());
+                d.halo = A.upload(t.halo.data(), t.halo.size());
+                d.ref = reinterpret_cast<const ushort4*>(A.upload(t.ref.data(), t.ref.size()));
+                d.pushAt = A.upload(t.pushAt.data(), t.pushAt.size());
+                d.push = A.upload(t.push.data(), t.push.size());
+                chunks_ = d;
+                return;
+            }
+            if (want == kSweepClusterChunks) return;
+            want = kSweepClusterChunks;
+        }
+    }
+    Arena chunkArena_;
+    SweepChunksDev chunks_;  // chunks = 0: a launch per sweep
+    int chunkKey_ = 0;
+
     void ensureMixedBuffers() {
         if (precision_ != AXISIM_PREC_MIXED && !fp32PressureCycle()) return;
         PhaseTimer ph(*this, "mixed_buffers");
@@ -2023,11 +2088,27 @@ private:
         }
     }
 
+    // Sweeps of the systems that fit the chip run in one launch each, unless the
+    // caller asked for tiles; the per-kernel profile keeps a launch per sweep, so
+    // that each has its own events.
+    bool onChip() const { return chunks_.chunks > 0 && tiles_.nTiles == 0 && !profiling_; }
+
     // The linear solver of one system (LinearSolver::run); `tag` names its
     // launches in the profile ("pp" or the scalar's).
     void enqueueLinear(double* x, double* xT, const double* AF, const double* b, const double* inv,
                        const char* tag = "pp") {
         const int iters = cs_.linearMaxIter;
+        {
+            SweepSystem<double, 1> a;
+            a.N = N_;
+            a.AF = AF;
+            a.b[0] = b;
+            a.inv[0] = inv;
+            a.x[0] = x;
+            if (onChip() && launchSweepChunks<double, 1>(ctl_, chunks_, a, iters, cs_.type == 1 ? colorN_ : 0, stream_)) {
+                return;
+            }
+        }
         if (cs_.type == 1 && colorN_ > 0) {
             for (int k = 0; k < iters; k++)
                 for (int c = 0; c < colorN_; c++) {
@@ -2125,7 +2206,16 @@ private:
         }
         // momentum solves (LinearSolver::run for u then v; fused, identical arithmetic)
         const int iters = cs_.linearMaxIter;
-        if (cs_.type == 1 && colorN_ > 0) {
+        SweepSystem<double, 2> uv;
+        uv.N = N_;
+        uv.AF = AFm_;
+        uv.b[0] = bu_; uv.b[1] = bv_;
+        uv.inv[0] = iu_; uv.inv[1] = iv_;
+        uv.x[0] = u_; uv.x[1] = v_;
+        if (!mixedMomentum && onChip() &&
+            launchSweepChunks<double, 2>(ctl_, chunks_, uv, iters, cs_.type == 1 ? colorN_ : 0, stream_)) {
+            // every sweep in that launch
+        } else if (cs_.type == 1 && colorN_ > 0) {
             for (int k = 0; k < iters; k++)
                 for (int c = 0; c < colorN_; c++) {
                     const int b0 = hColorStart_[(size_t)c], cnt = hColorStart_[(size_t)c + 1] - b0;
@@ -2141,7 +2231,17 @@ private:
             mark("ir_residual_uv", (double)N_ * (8.0 * W_ + 64.0 + 24.0) + meshSlotIndexBytes());
             int c = 0;
             const int rest = iters - 1;
-            if (tiles_.nTiles > 0 && rest > 1) {
+            SweepSystem<float, 2> duv;
+            duv.N = N_;
+            duv.AF = AF32m_;
+            duv.b[0] = ru32_; duv.b[1] = rv32_;
+            duv.inv[0] = iu32_; duv.inv[1] = iv32_;
+            duv.x[0] = du32_[0]; duv.x[1] = dv32_[0];
+            duv.addTo[0] = u_; duv.addTo[1] = v_;
+            bool added = false;  // the sweeps' launch also applied the correction
+            if (onChip() && launchSweepChunks<float, 2>(ctl_, chunks_, duv, rest, 0, stream_)) {
+                added = true;
+            } else if (tiles_.nTiles > 0 && rest > 1) {
                 // the remaining sweeps in launches of at most S, as even as possible
                 const int L = (rest + tiles_.S - 1) / tiles_.S;
                 for (int q = 0; q < L; q++) {
@@ -2159,8 +2259,10 @@ private:
                     c = 1 - c;
                 }
             }
-            launchIRUpdateUV(ctl_, N_, u_, v_, du32_[c], dv32_[c], stream_);
-            mark("ir_update_uv", 40.0 * N_);
+            if (!added) {
+                launchIRUpdateUV(ctl_, N_, u_, v_, du32_[c], dv32_[c], stream_);
+                mark("ir_update_uv", 40.0 * N_);
+            }
         } else {
             double *lu = u_, *su = uT_, *lv = v_, *sv = vT_;
             if (tiles_.nTiles > 0 && iters > 1) {
@@ -2505,6 +2607,7 @@ private:
         if (cs_.useMultigrid && psolve_ == AXISIM_PSOLVE_FCG) ensureNetStats();
         if (cs_.type == 1) ensureColoring();
         ensureSweepTiles();
+        ensureSweepChunks();
         if (autotune_ && cs_.useMultigrid) {  // launch shapes are fixed in the graph: tune first
             if (fp32PressureCycle()) {
                 if (!levels32_.empty() && levels32_[0].block == 0) tuneLevels(levels32_);

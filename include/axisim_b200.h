@@ -258,7 +258,8 @@ int axisim_pressure_stats(axisim_handle* h, int64_t* solves, int64_t* iterations
 int axisim_set_vcycle_kernel(axisim_handle* h, int32_t mode);
 /* New (the reference launches one kernel per Jacobi sweep of each momentum
  * component, linear_solver.cu:91-146): how many of the u/v momentum Jacobi
- * sweeps one launch runs (1..8, default 1). Above 1 the cells are cut into
+ * sweeps one launch runs (1..8, default 1; a mesh of at most 16,384 cells then
+ * runs all of them in one launch on the chip). Above 1 the cells are cut into
  * tiles along a space-filling curve of their centres; a launch loads a
  * tile's coefficients once, keeps the iterate of the tile and its halo in
  * shared memory and repeats the sweep there, each sweep on a halo one layer
@@ -450,7 +451,9 @@ typedef struct axisim_kernel_stat {
 } axisim_kernel_stat;
 /* New (the reference times only the whole solve, solver.cpp:907-908,1318-1323):
  * runs `iterations` SIMPLE iterations eagerly from the current state, with an
- * event recorded after every kernel on the solver's stream. */
+ * event recorded after every kernel on the solver's stream. The linear sweeps
+ * that a solve runs in one launch (systems that fit the chip) are launched one
+ * by one here, with the same results. */
 int axisim_profile_iteration(axisim_handle* h, int32_t iterations, axisim_kernel_stat* out, int32_t maxOut,
                              int32_t* nOut);
 /* As axisim_profile_iteration, with every multigrid launch (smoothing,
