@@ -214,7 +214,6 @@ constexpr int kSweepK64 = 2;
 constexpr int kMaxSweepsPerLaunch = 8;
 
 // ---- one SIMPLE iteration ----
-void launchIterBegin(Ctl* ctl, const volatile int* hostStop, cudaStream_t s);
 // gradients of up to five fields (u, v, p, T, C) with their boundary fields
 void launchGradient(const MeshDev& m, const Ctl* ctl, int nFields, const double* const* phi, const BCDev* bc,
                     double* const* gZ, double* const* gR, int scheme, cudaStream_t s);
@@ -255,10 +254,12 @@ void launchResiduals(const MeshDev& m, const Ctl* ctl, const double* AF, const d
                      int* nBlocksOut, cudaStream_t s);
 // partialS: per block {stat_T, |diag_T|, stat_C, |diag_C|} of the scalar
 // residual pass (null when no scalar residual is monitored)
-void launchIterEnd(Ctl* ctl, const double* partial, const double* partialS, int nBlocks, int N, cudaStream_t s);
+// and the next iteration's checks: a stop request (hostStop), the iteration limit
+void launchIterEnd(Ctl* ctl, const double* partial, const double* partialS, int nBlocks, int N,
+                   const volatile int* hostStop, cudaStream_t s);
 // batch: per-case reduction of the per-cell residual arrays, then per-case norms + convergence
 void launchBatchIterEnd(Ctl* ctl, const BatchDev& b, const double* resU, const double* resV, const double* resC,
-                        const double* scaleU, const double* scaleV, cudaStream_t s);
+                        const double* scaleU, const double* scaleV, const volatile int* hostStop, cudaStream_t s);
 void launchCopy(const Ctl* ctl, double* dst, const double* src, int n, cudaStream_t s);
 
 // ---- transported scalars (scalar.cu) ----

@@ -182,22 +182,18 @@ __global__ void k_build_seg(int N, int W, const int32_t* __restrict__ snb, const
 }
 
 // ---------------- iteration control ----------------
-__global__ void k_iter_begin(Ctl* ctl, const volatile int* hostStop) {
-    pdlEnter();
-    if (ctl->done) return;
-    if (hostStop && *hostStop) {
-        ctl->done = 2;
-        return;
+// The end of an iteration decides about the next one: one that must not run ends
+// the solve, so the host replays exactly maxIter graphs and no iteration opens
+// with a launch of its own. `stop`: the host's stop request, as the iteration's
+// last kernel read it when it started.
+__device__ __forceinline__ void iterNext(Ctl* ctl, int done, int k, int stop, int mgErr, int maxIter, int checkConv) {
+    if (!done) {
+        if (stop) done = 2;
+        else if (mgErr) done = 5;  // a grid barrier of the resident V-cycle gave up
+        else if (k >= maxIter) done = 3;
+        else ctl->checked = k % checkConv == 0;
     }
-    if (ctl->mgErr) {  // a grid barrier of the resident V-cycle gave up
-        ctl->done = 5;
-        return;
-    }
-    if (ctl->k >= ctl->maxIter) {
-        ctl->done = 3;
-        return;
-    }
-    ctl->checked = (ctl->k % ctl->checkConv) == 0;
+    if (done) ctl->done = done;
 }
 
 // ---------------- gradients (solver_util.cu:146-169, cuh:458-588) ----------------
@@ -1000,104 +996,145 @@ __global__ void __launch_bounds__(kThreads) k_residual(MeshDev m, const Ctl* ctl
 // + iteration counters, all on the device (no host synchronisation).
 constexpr int kResS = 4;  // stat_T, |diag_T|, stat_C, |diag_C|
 
+// The sum (or maximum) of one statistic over the blocks' partials: thread t of
+// 256 takes the blocks t, t + 256, ..., 16 loads ahead, and the threads combine
+// as a tree over 256 does (t with t + 128, t + 64, ..., t + 1). One statistic
+// per warp after the first pass, so the tree needs one barrier.
+template <int NQ>
+__device__ __forceinline__ void blockColumns(const double* __restrict__ partial, int nBlocks, const bool (&isMax)[NQ],
+                                             double (*sh)[kThreads]) {
+    double acc[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) acc[q] = isMax[q] ? -INFINITY : 0.0;
+    constexpr int kAhead = 16;
+    for (int i = threadIdx.x; i < nBlocks; i += kAhead * kThreads) {
+        double v[kAhead][NQ];
+#pragma unroll
+        for (int u = 0; u < kAhead; u++)
+#pragma unroll
+            for (int q = 0; q < NQ; q++) v[u][q] = partial[(size_t)min(i + u * kThreads, nBlocks - 1) * NQ + q];
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+            if (i + u * kThreads >= nBlocks) break;
+#pragma unroll
+            for (int q = 0; q < NQ; q++) acc[q] = combine(acc[q], v[u][q], isMax[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; q++) sh[q][threadIdx.x] = acc[q];
+}
+
 __global__ void __launch_bounds__(kThreads) k_iter_end(Ctl* ctl, const double* partial, const double* partialS,
-                                                       int nBlocks, int N) {
+                                                       int nBlocks, int N, const volatile int* hostStop) {
+    const int stop = threadIdx.x == 0 && hostStop ? *hostStop : 0;  // host memory: on its way while this waits
     pdlEnter();
     if (ctl->done) return;
     constexpr int NQ = kResQ + kResS;
-    __shared__ double sh[kThreads][NQ];
-    if (ctl->checked) {
-        const int isMax[NQ] = {ctl->resNorm[0] == 2, 0, ctl->resNorm[1] == 2, 0, 0,
-                               ctl->resNormS[0] == 2, 0, ctl->resNormS[1] == 2, 0};
-        double acc[NQ];
-        for (int q = 0; q < NQ; q++) acc[q] = isMax[q] ? -INFINITY : 0.0;
-#pragma unroll 4
-        for (int i = threadIdx.x; i < nBlocks; i += blockDim.x) {  // unrolled: the loads of four rows in flight
-            for (int q = 0; q < kResQ; q++) acc[q] = combine(acc[q], partial[(size_t)i * kResQ + q], isMax[q]);
-            if (partialS)
-                for (int q = 0; q < kResS; q++)
-                    acc[kResQ + q] = combine(acc[kResQ + q], partialS[(size_t)i * kResS + q], isMax[kResQ + q]);
+    __shared__ double sh[NQ][kThreads];
+    __shared__ double total[NQ];
+    // the control block's entries that thread 0 decides on, loaded together
+    const bool checked = ctl->checked != 0;
+    int k = 0, iteration = 0, calls = 0, mgErr = 0, maxIter = 0, checkConv = 1, transient = 0, hist = 0;
+    int enabled[5], norm[5], scale[5], solved[2];
+    double tol[5], scaleVal[5], resVal[5];
+    if (threadIdx.x == 0) {
+        k = ctl->k;
+        iteration = ctl->currentIteration;
+        calls = ctl->itersThisCall;
+        mgErr = ctl->mgErr;
+        maxIter = ctl->maxIter;
+        checkConv = ctl->checkConv;
+        transient = ctl->transient;
+        hist = ctl->histCount;
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+            enabled[i] = i < 3 ? ctl->resEnabled[i] : ctl->resEnabledS[i - 3];
+            norm[i] = i < 3 ? ctl->resNorm[i] : ctl->resNormS[i - 3];
+            scale[i] = i < 3 ? ctl->resScale[i] : ctl->resScaleS[i - 3];
+            tol[i] = i < 3 ? ctl->tol[i] : ctl->tolS[i - 3];
+            scaleVal[i] = i < 3 ? ctl->scaleVal[i] : ctl->scaleValS[i - 3];
+            resVal[i] = i < 3 ? ctl->resVal[i] : ctl->resValS[i - 3];
         }
-        for (int q = 0; q < NQ; q++) sh[threadIdx.x][q] = acc[q];
+        solved[0] = ctl->solvedS[0];
+        solved[1] = ctl->solvedS[1];
+    }
+    if (checked) {
+        const bool maxU = ctl->resNorm[0] == 2, maxV = ctl->resNorm[1] == 2;
+        const bool maxT = ctl->resNormS[0] == 2, maxC = ctl->resNormS[1] == 2;
+        {
+            const bool isMax[kResQ] = {maxU, false, maxV, false, false}, none[kResQ] = {};
+            if (maxU || maxV) blockColumns<kResQ>(partial, nBlocks, isMax, sh);
+            else blockColumns<kResQ>(partial, nBlocks, none, sh);
+        }
+        if (partialS) {
+            const bool isMax[kResS] = {maxT, false, maxC, false};
+            blockColumns<kResS>(partialS, nBlocks, isMax, sh + kResQ);
+        }
         __syncthreads();
-        for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-            if ((int)threadIdx.x < st)
-                for (int q = 0; q < NQ; q++)
-                    sh[threadIdx.x][q] = combine(sh[threadIdx.x][q], sh[threadIdx.x + st][q], isMax[q]);
-            __syncthreads();
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        for (int q = warp; q < (partialS ? NQ : kResQ); q += kThreads / 32) {
+            const bool isMax = (q == 0 && maxU) || (q == 2 && maxV) || (q == kResQ && maxT) || (q == kResQ + 2 && maxC);
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = sh[q][lane + 32 * u];
+#pragma unroll
+            for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (u < h) v[u] = combine(v[u], v[u + h], isMax);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[0] = combine(v[0], __shfl_down_sync(0xffffffffu, v[0], o), isMax);
+            if (lane == 0) total[q] = v[0];
         }
+        __syncthreads();
     }
     if (threadIdx.x != 0) return;
-    if (ctl->checked) {
-        const double raw[3] = {sh[0][0], sh[0][2], sh[0][4]};
-        const double diag[2] = {sh[0][1], sh[0][3]};
-        const int scaleIteration = ctl->transient ? ctl->k : ctl->currentIteration;
-        for (int i = 0; i < 3; i++) {
-            if (!ctl->resEnabled[i]) continue;
-            ctl->resVal[i] = raw[i];
-            if (i < 2) {
-                switch (ctl->resScale[i]) {
-                    case 0: ctl->scaleVal[i] = 1.0; break;
-                    case 1: ctl->scaleVal[i] = (double)N; break;
-                    case 2: ctl->scaleVal[i] = sqrt((double)N); break;
-                    case 3: ctl->scaleVal[i] = diag[i]; break;
+    int done = 0;
+    if (checked) {
+        const int scaleIteration = transient ? k : iteration;
+        bool any = false, conv = true, finite = true;
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+            if (!enabled[i]) continue;
+            // Temperature and Concentration entries: an unsolved scalar's system is all zero
+            const int q = i < 2 ? 2 * i : i == 2 ? 4 : kResQ + 2 * (i - 3);
+            const bool zero = i >= 3 && !(partialS && solved[i >= 3 ? i - 3 : 0]);
+            double r = zero ? 0.0 : total[q];
+            if (i != 2) {
+                switch (scale[i]) {
+                    case 0: scaleVal[i] = 1.0; break;
+                    case 1: scaleVal[i] = (double)N; break;
+                    case 2: scaleVal[i] = sqrt((double)N); break;
+                    case 3: scaleVal[i] = zero ? 0.0 : total[q + 1]; break;
                     default: break;
                 }
+            } else if (scaleIteration < 5) {
+                scaleVal[i] = fmax(r, 0.0);
             }
-        }
-        bool finite = true;
-        for (int i = 0; i < 3; i++) {
-            if (!ctl->resEnabled[i]) continue;
-            if (i == 2 && scaleIteration < 5) ctl->scaleVal[i] = fmax(ctl->resVal[i], 0.0);
-            if (ctl->scaleVal[i] == 0.0) continue;
-            if (ctl->resNorm[i] == 1) ctl->resVal[i] = sqrt(ctl->resVal[i]);
-            ctl->resVal[i] /= ctl->scaleVal[i];
-        }
-        // Temperature and Concentration entries (an unsolved scalar's system is all zero)
-        for (int e = 0; e < 2; e++) {
-            if (!ctl->resEnabledS[e]) continue;
-            const double raw = ctl->solvedS[e] ? sh[0][kResQ + 2 * e] : 0.0;
-            const double diag = ctl->solvedS[e] ? sh[0][kResQ + 2 * e + 1] : 0.0;
-            ctl->resValS[e] = raw;
-            switch (ctl->resScaleS[e]) {
-                case 0: ctl->scaleValS[e] = 1.0; break;
-                case 1: ctl->scaleValS[e] = (double)N; break;
-                case 2: ctl->scaleValS[e] = sqrt((double)N); break;
-                case 3: ctl->scaleValS[e] = diag; break;
-                default: break;
+            if (scaleVal[i] != 0.0) {
+                if (norm[i] == 1) r = sqrt(r);
+                r /= scaleVal[i];
             }
-            if (ctl->scaleValS[e] == 0.0) continue;
-            if (ctl->resNormS[e] == 1) ctl->resValS[e] = sqrt(ctl->resValS[e]);
-            ctl->resValS[e] /= ctl->scaleValS[e];
-        }
-        bool any = false, conv = true;
-        for (int i = 0; i < 3; i++) {
-            if (!ctl->resEnabled[i]) continue;
+            resVal[i] = r;
             any = true;
-            if (!(ctl->resVal[i] <= ctl->tol[i])) conv = false;
-            if (!isfinite(ctl->resVal[i])) finite = false;
-        }
-        for (int e = 0; e < 2; e++) {
-            if (!ctl->resEnabledS[e]) continue;
-            any = true;
-            if (!(ctl->resValS[e] <= ctl->tolS[e])) conv = false;
-            if (!isfinite(ctl->resValS[e])) finite = false;
+            if (!(r <= tol[i])) conv = false;
+            if (!isfinite(r)) finite = false;
+            (i < 3 ? ctl->resVal[i] : ctl->resValS[i - 3]) = r;
+            (i < 3 ? ctl->scaleVal[i] : ctl->scaleValS[i - 3]) = scaleVal[i];
         }
         ctl->converged = any && conv;
-        const int h = ctl->histCount % kMaxHist;
-        ctl->hist[h][0] = (double)ctl->currentIteration;
-        ctl->hist[h][1] = ctl->resVal[0];
-        ctl->hist[h][2] = ctl->resVal[1];
-        ctl->hist[h][3] = ctl->resVal[2];
-        ctl->hist[h][4] = ctl->resValS[0];
-        ctl->hist[h][5] = ctl->resValS[1];
-        ctl->histCount++;
-        if (ctl->converged) ctl->done = 1;
-        else if (!finite) ctl->done = 4;
+        double* h = ctl->hist[hist % kMaxHist];
+        h[0] = (double)iteration;
+#pragma unroll
+        for (int i = 0; i < 5; i++) h[1 + i] = resVal[i];
+        ctl->histCount = hist + 1;
+        if (any && conv) done = 1;
+        else if (!finite) done = 4;
     }
-    ctl->k++;
-    ctl->currentIteration++;
-    ctl->itersThisCall++;
+    ctl->k = k + 1;
+    ctl->currentIteration = iteration + 1;
+    ctl->itersThisCall = calls + 1;
+    iterNext(ctl, done, k + 1, stop, mgErr, maxIter, checkConv);
 }
 
 // Sums over a case's cell range of the per-cell residual arrays k_residual
@@ -1148,7 +1185,8 @@ __global__ void __launch_bounds__(kThreads) k_case_reduce(const Ctl* ctl, BatchD
 
 // residualAllHost's arithmetic and the convergence test, case by case; the
 // batch is done once every case has converged.
-__global__ void __launch_bounds__(kThreads) k_batch_iter_end(Ctl* ctl, BatchDev b, int N) {
+__global__ void __launch_bounds__(kThreads) k_batch_iter_end(Ctl* ctl, BatchDev b, const volatile int* hostStop) {
+    const int stop = threadIdx.x == 0 && hostStop ? *hostStop : 0;
     pdlEnter();
     if (ctl->done) return;
     __shared__ int nConv, nBad;
@@ -1200,6 +1238,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_iter_end(Ctl* ctl, BatchDev 
     }
     __syncthreads();
     if (threadIdx.x != 0) return;
+    int done = 0;
     if (ctl->checked) {
         ctl->casesConverged = nConv;
         ctl->converged = nConv == b.nCases;
@@ -1212,13 +1251,14 @@ __global__ void __launch_bounds__(kThreads) k_batch_iter_end(Ctl* ctl, BatchDev 
         ctl->hist[h][4] = 0.0;
         ctl->hist[h][5] = 0.0;
         ctl->histCount++;
-        if (ctl->converged) ctl->done = 1;
-        else if (nBad) ctl->done = 4;
+        if (ctl->converged) done = 1;
+        else if (nBad) done = 4;
     }
-    ctl->k++;
+    const int k = ctl->k + 1;
+    ctl->k = k;
     ctl->currentIteration++;
     ctl->itersThisCall++;
-    (void)N;
+    iterNext(ctl, done, k, stop, ctl->mgErr, ctl->maxIter, ctl->checkConv);
 }
 
 __global__ void k_copy(const Ctl* ctl, double* dst, const double* src, int n) {
@@ -1250,10 +1290,6 @@ void launchBuildEll(int N, int W, const int32_t* cfs, const int32_t* cfi, const 
 void launchBuildSegments(const MeshDev& m, int4* seg, int4* segF, int* segM, int* nIrregular, cudaStream_t s) {
     launchPDL(k_build_seg, dim3(blocksFor((m.N + 31) / 32)), dim3(kThreads), 0, s, m.N, m.W, m.snb, m.sface, m.owner,
               m.neighbor, seg, segF, segM, nIrregular);
-}
-
-void launchIterBegin(Ctl* ctl, const volatile int* hostStop, cudaStream_t s) {
-    launchPDL(k_iter_begin, dim3(1), dim3(1), 0, s, ctl, hostStop);
 }
 
 void launchGradient(const MeshDev& m, const Ctl* ctl, int nFields, const double* const* phi, const BCDev* bc,
@@ -1371,14 +1407,15 @@ void launchResiduals(const MeshDev& m, const Ctl* ctl, const double* AF, const d
                                       partial);
 }
 
-void launchIterEnd(Ctl* ctl, const double* partial, const double* partialS, int nBlocks, int N, cudaStream_t s) {
-    launchPDL(k_iter_end, dim3(1), dim3(kThreads), 0, s, ctl, partial, partialS, nBlocks, N);
+void launchIterEnd(Ctl* ctl, const double* partial, const double* partialS, int nBlocks, int N,
+                   const volatile int* hostStop, cudaStream_t s) {
+    launchPDL(k_iter_end, dim3(1), dim3(kThreads), 0, s, ctl, partial, partialS, nBlocks, N, hostStop);
 }
 
 void launchBatchIterEnd(Ctl* ctl, const BatchDev& b, const double* resU, const double* resV, const double* resC,
-                        const double* scaleU, const double* scaleV, cudaStream_t s) {
+                        const double* scaleU, const double* scaleV, const volatile int* hostStop, cudaStream_t s) {
     launchPDL(k_case_reduce, dim3(b.nCases, kResQ), dim3(kThreads), 0, s, ctl, b, resU, resV, resC, scaleU, scaleV);
-    launchPDL(k_batch_iter_end, dim3(1), dim3(kThreads), 0, s, ctl, b, 0);
+    launchPDL(k_batch_iter_end, dim3(1), dim3(kThreads), 0, s, ctl, b, hostStop);
 }
 
 void launchCopy(const Ctl* ctl, double* dst, const double* src, int n, cudaStream_t s) {

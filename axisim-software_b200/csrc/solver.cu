@@ -2162,8 +2162,6 @@ private:
         const int nonOrtho = cs_.useNonOrthCorrector ? 1 : 0;
         const bool convNeedsGrad = conv && (scheme == 2 || scheme == 3);
         const int grad = cs_.gradientScheme;
-        launchIterBegin(ctl_, hostStopDev_, stream_);
-        mark("iter_begin", 0.0);
         // gradients of u, v (when SOU / non-orthogonal) and p in one pass; the
         // solved scalars' gradients join it: the reference takes them just
         // before each scalar's assembly (solver.cpp:1224-1226), and nothing
@@ -2403,10 +2401,10 @@ private:
             mark("scalar_residual", ns * (8.0 * W_ + 48.0) * N_ + 4.0 * W_ * N_);
         }
         if (batch_.nCases > 0) {
-            launchBatchIterEnd(ctl_, batch_, resU_, resV_, resC_, scU_, scV_, stream_);
+            launchBatchIterEnd(ctl_, batch_, resU_, resV_, resC_, scU_, scV_, hostStopDev_, stream_);
             mark("batch_iter_end", 40.0 * N_);
         } else {
-            launchIterEnd(ctl_, partial_, monitorS ? partialS_ : nullptr, residualBlocks_, N_, stream_);
+            launchIterEnd(ctl_, partial_, monitorS ? partialS_ : nullptr, residualBlocks_, N_, hostStopDev_, stream_);
             mark("iter_end", 40.0 * residualBlocks_);
         }
     }
@@ -2429,6 +2427,7 @@ public:
         CK(cudaMemcpy(&h, ctl_, sizeof(Ctl), cudaMemcpyDeviceToHost));
         const Ctl saved = h;
         h.done = 0;
+        h.checked = 1;
         h.k = 0;
         h.maxIter = 1 << 30;
         h.checkConv = std::max(1, csim_.checkConv);
@@ -2805,7 +2804,10 @@ int Solver::solve(int continueRun, axisim_result* res) {
                 CK(cudaMemcpyAsync(b.old(), b.phi, (size_t)N_ * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
             }
         }
-        h.done = 0;
+        // the first iteration of a step is decided here, each later one by the
+        // end of the one before it (k_iter_end)
+        h.done = __atomic_load_n(hostStop_, __ATOMIC_SEQ_CST) ? 2 : 0;
+        h.checked = 1;
         h.k = 0;
         h.bdf2 = (bdf2 && t > 0) ? 1 : 0;
         h.converged = 0;
@@ -2815,8 +2817,8 @@ int Solver::solve(int continueRun, axisim_result* res) {
         int batch = 4;
         int launched = 0;
         int drained = 0;
-        for (;;) {
-            const int nb = std::min(batch, std::max(1, csim_.maxIter - launched + 1));
+        while (!h.done) {
+            const int nb = std::min(batch, std::max(1, csim_.maxIter - launched));
             for (int i = 0; i < nb; i++) CK(cudaGraphLaunch(exec_, stream_));
             launched += nb;
             CK(cudaMemcpyAsync(&h, ctl_, sizeof(Ctl), cudaMemcpyDeviceToHost, stream_));
@@ -2828,7 +2830,6 @@ int Solver::solve(int continueRun, axisim_result* res) {
                 }
             }
             drained = h.histCount;
-            if (h.done) break;
             batch = std::min(batch * 2, 64);
         }
         totalIters += h.itersThisCall - startIters;
