@@ -281,8 +281,7 @@ void launchScalarResidual(const MeshDev& m, const Ctl* ctl, int ns, int first, c
 template <class TF, class TC>
 void launchGalerkin(const Ctl* ctl, const LevelT<TF>& fine, const LevelT<TC>& coarse, cudaStream_t s);
 // Galerkin of a chain of small levels (lv[i] -> lv[i+1], i < count - 1) in one
-// single-CTA launch, level by level: the coarse operators of the V-cycle
-// tail, each at most 1024 cells, without a launch per level.
+// launch of one cluster, level by level, without a launch per level.
 template <class T>
 struct GalChainArgsT {
     int count = 0;

@@ -18,6 +18,8 @@
 // inner cycles of the mixed-precision path.
 #include <cmath>
 
+#include <cooperative_groups.h>
+
 #include "coarsest.cuh"
 #include "kernels.hpp"
 
@@ -28,6 +30,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kTailThreads = 1024;  // tail levels hold at most this many cells: one row per thread
 constexpr int kRegW = 16;
+constexpr int kGalCtas = 8, kGalThreads = 512;  // the deep levels' Galerkin
 
 inline int blocksFor(long long n, int t = kThreads) { return (int)((n + t - 1) / t); }
 // Threads per CTA for a level's kernels: its tuned block size, else kThreads
@@ -525,7 +528,15 @@ template <class TF, class TC, bool NC>
 __device__ __forceinline__ void galCoarseCell(const LevelT<TF>& F, const LevelT<TC>& C, int t) {
     if (t < C.totalSlots) {
         TF af = TF(0);
-        for (int q = C.gStart[t]; q < C.gStart[t + 1]; q++) af += F.AF[C.gList[q]];
+        const int q0 = C.gStart[t], q1 = C.gStart[t + 1];
+        for (int q = q0; q < q1; q += 4) {  // four feeding slots' loads at once, summed in order
+            TF v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = F.AF[C.gList[min(q + u, q1 - 1)]];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (q + u < q1) af += v[u];
+        }
         C.AF[t] = (TC)af;
     }
     if (t < C.N) {
@@ -550,19 +561,28 @@ __global__ void __launch_bounds__(kThreads) k_gal_coarse(const Ctl* ctl, LevelT<
     galCoarseCell<TF, TC, true>(F, C, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// The tail levels' Galerkin in one CTA: a coarse level's operator is read as
-// the next pair's fine level after the barrier (plain loads: it was written
-// in this launch).
+// The deep levels' Galerkin in one launch of one cluster: a coarse level's
+// operator is read as the next pair's fine level after the cluster barrier
+// (plain loads: it was written in this launch). A level is two or three
+// dependent loads, so a chain costs a load chain and a barrier per level, not a
+// launch; one CTA of 1,024 threads took 25-30 us for it, and the first V-cycle
+// waited for that. Whole runs against the single CTA: 874k cells mixed 15.82 ->
+// 15.44 ms for 20 iterations, FP64 9.40 -> 9.03 for 10, 53k mixed 8.45 -> 8.19 for
+// 40; a launch per level measured 15.44, 9.08 and 8.20 (8,000 cells: 10.49
+// against 10.18), 256 threads 15.49, 9.06 and 8.3, and a chain from 4,096 cells on
+// 15.58, 9.08 and 8.29: the larger levels want more than eight SMs.
 template <class T>
-__global__ void __launch_bounds__(kTailThreads) k_gal_chain(const Ctl* ctl, GalChainArgsT<T> a) {
+__global__ void __launch_bounds__(kGalThreads) k_gal_chain(const Ctl* ctl, GalChainArgsT<T> a) {
+    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     pdlEnter();
-    if (ctl->done || ctl->ppSkip) return;
+    if (ctl->done || ctl->ppSkip) return;  // the same on every CTA
     for (int i = 0; i + 1 < a.count; i++) {
         const LevelT<T>& F = a.lv[i];
         const LevelT<T>& C = a.lv[i + 1];
         const int n = C.totalSlots > C.N ? C.totalSlots : C.N;
-        for (int t = threadIdx.x; t < n; t += blockDim.x) galCoarseCell<T, T, false>(F, C, t);
-        __syncthreads();
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+            galCoarseCell<T, T, false>(F, C, t);
+        if (i + 2 < a.count) cl.sync();
     }
 }
 
@@ -847,7 +867,29 @@ void launchGalerkin(const Ctl* ctl, const LevelT<TF>& fine, const LevelT<TC>& co
 
 template <class T>
 void launchGalerkinChain(const Ctl* ctl, const GalChainArgsT<T>& a, cudaStream_t s) {
-    launchPDL(k_gal_chain<T>, dim3(1), dim3(kTailThreads), 0, s, ctl, a);
+    // a cluster of kGalCtas CTAs (portable size); one CTA where a device refuses it
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kGalCtas);
+    cfg.blockDim = dim3(kGalThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kGalCtas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_gal_chain<T>, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        launchPDL(k_gal_chain<T>, dim3(1), dim3(kGalThreads), 0, s, ctl, a);
+        return;
+    }
+    cfg.numAttrs = tNextLaunchPlain ? 1 : 2;
+    tNextLaunchPlain = false;
+    cudaLaunchKernelEx(&cfg, k_gal_chain<T>, ctl, a);
 }
 
 template <class T>

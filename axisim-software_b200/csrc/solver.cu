@@ -1879,7 +1879,7 @@ private:
     }
 
     // The Galerkin steps into the tail levels (at most 1024 cells each) run in
-    // one single-CTA launch; returns the first coarse level of that chain (L:
+    // one cluster launch; returns the first coarse level of that chain (L:
     // none). The chain starts at level 2 or deeper, so its first fine level is
     // one of the cycle's own levels in either precision.
     int galerkinChainStart(int L) const {
