@@ -32,7 +32,7 @@ namespace axisim {
 namespace {
 
 constexpr int kThreads = 256;
-inline int blocksFor(int n) { return (n + kThreads - 1) / kThreads; }
+inline int blocksFor(int n, int rows = 1) { return (n + kThreads * rows - 1) / (kThreads * rows); }
 
 __device__ __forceinline__ double opAx(const LevelDev& L, int n, const double* __restrict__ x) {
     double Ax = L.AC[n] * x[n];
@@ -44,33 +44,39 @@ __device__ __forceinline__ double opAx(const LevelDev& L, int n, const double* _
     return Ax;
 }
 
-// Block sums of NQ values -> partial[block][NQ]; the last block to arrive adds
-// all partials in block order and writes out[0..NQ). counter starts at 0 and is
-// returned to 0 by the last block.
+// Sums of NQ values over groups of 256 cells -> partial[group][NQ], G groups a
+// block (the block's rows are loaded together: more loads in flight, and one
+// arrival for G groups); the last block to arrive adds all partials in group
+// order, 16 loads ahead of its sums, and writes out[0..NQ). The order of every
+// sum is that of one group a block, so G changes no bit. counter starts at 0
+// and is returned to 0 by the last block.
 // Returns true in thread 0 of the last block, after out[] is written.
-template <int NQ>
-__device__ __forceinline__ bool gridSum(const double (&v)[NQ], double* __restrict__ partial,
+template <int NQ, int G>
+__device__ __forceinline__ bool gridSum(const double (&v)[G][NQ], int N, double* __restrict__ partial,
                                         unsigned int* counter, double* out) {
-    __shared__ double sh[kThreads / 32][NQ];
+    __shared__ double sh[G][kThreads / 32][NQ];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int groups = (N + kThreads - 1) / kThreads;
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
-        double x = v[q];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0) sh[warp][q] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    for (int u = 0; u < G; u++)
 #pragma unroll
         for (int q = 0; q < NQ; q++) {
-            double x = 0.0;
-            for (int w = 0; w < kThreads / 32; w++) x += sh[w][q];
-            partial[(size_t)blockIdx.x * NQ + q] = x;
+            double x = v[u][q];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+            if (lane == 0) sh[u][warp][q] = x;
         }
+    __syncthreads();
+    if (threadIdx.x < G * NQ) {
+        const int u = threadIdx.x / NQ, q = threadIdx.x % NQ, g = blockIdx.x * G + u;
+        double x = 0.0;
+        for (int w = 0; w < kThreads / 32; w++) x += sh[u][w][q];
+        if (g < groups) partial[(size_t)g * NQ + q] = x;
         __threadfence();
-        last = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return false;
     __threadfence();
@@ -78,9 +84,19 @@ __device__ __forceinline__ bool gridSum(const double (&v)[NQ], double* __restric
 #pragma unroll
     for (int q = 0; q < NQ; q++) acc[q] = 0.0;
     // fixed assignment of partials to threads and a fixed tree: deterministic
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads)
+    constexpr int kAhead = 16;
+    for (int i = threadIdx.x; i < groups; i += kAhead * kThreads) {
+        double x[kAhead][NQ];
 #pragma unroll
-        for (int q = 0; q < NQ; q++) acc[q] += ((volatile double*)partial)[(size_t)i * NQ + q];
+        for (int u = 0; u < kAhead; u++)
+#pragma unroll
+            for (int q = 0; q < NQ; q++) x[u][q] = __ldcg(partial + (size_t)min(i + u * kThreads, groups - 1) * NQ + q);
+#pragma unroll
+        for (int u = 0; u < kAhead; u++)
+            if (i + u * kThreads < groups)
+#pragma unroll
+                for (int q = 0; q < NQ; q++) acc[q] += x[u][q];
+    }
     __shared__ double tr[kThreads][NQ];
 #pragma unroll
     for (int q = 0; q < NQ; q++) tr[threadIdx.x][q] = acc[q];
@@ -110,7 +126,7 @@ __global__ void __launch_bounds__(kThreads) k_fcg_init(Ctl* ctl, LevelDev L, con
     pdlEnter();
     if (ctl->done) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    double acc[2] = {0.0, 0.0};
+    double acc[1][2] = {};
     if (n < L.N) {
         const double bv = L.b[n];
         const double rv = bv - opAx(L, n, x);
@@ -120,16 +136,24 @@ __global__ void __launch_bounds__(kThreads) k_fcg_init(Ctl* ctl, LevelDev L, con
             const double ac = L.AC[n];
             eFirst[n] = (fabs(ac) < 1.0e-30) ? 0.f : (float)(w * rv / ac);
         }
-        acc[0] = bv * bv;
-        acc[1] = rv * rv;
+        acc[0][0] = bv * bv;
+        acc[0][1] = rv * rv;
     }
-    if (gridSum<2>(acc, partial, counter, s + 4)) {
+    if (gridSum<2, 1>(acc, L.N, partial, counter, s + 4)) {
         ctl->ppSolves++;
         s[6] = (double)ctl->ppIterations;  // Krylov iterations before this solve
         s[7] = s[5];                       // (r0, r0)
         if (s[5] <= relTol * relTol * s[4]) ctl->ppSkip = 1;
     }
 }
+
+// Rows a thread takes in the passes below: their loads are in flight together.
+// 2M cells, us a launch in the per-kernel profile (some 4 us of them its events),
+// one row a thread and one partial at a time in the last block -> now: dots
+// 28.5 -> 20.5, update 40.3 -> 28.4, product 55.3 -> 47.3. A whole step with 90
+// iterations: 23.8 ms; 24.0 with two rows in the product, 24.3 with one in the
+// update, 24.0 with eight in the dots (each with two in the update), 26.4 before.
+constexpr int kDotRows = 4, kUpdateRows = 4, kSpmvRows = 1;
 
 // s[0] = (r, e), s[1] = (e, q_prev) (useQ) with e the V-cycle's output.
 __global__ void __launch_bounds__(kThreads) k_fcg_dots(const Ctl* ctl, int N, const float* __restrict__ e,
@@ -138,19 +162,31 @@ __global__ void __launch_bounds__(kThreads) k_fcg_dots(const Ctl* ctl, int N, co
                                                        double* s) {
     pdlEnter();
     if (ctl->done || ctl->ppSkip) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    double acc[2] = {0.0, 0.0};
-    if (n < N) {
-        const double z = (double)e[n];
-        acc[0] = r[n] * z;
-        if (useQ) acc[1] = z * q[n];
+    double acc[kDotRows][2] = {};
+    double ev[kDotRows], rv[kDotRows], qv[kDotRows];
+#pragma unroll
+    for (int u = 0; u < kDotRows; u++) {
+        const int n = min((blockIdx.x * kDotRows + u) * kThreads + (int)threadIdx.x, N - 1);
+        ev[u] = (double)e[n];
+        rv[u] = r[n];
+        qv[u] = useQ ? q[n] : 0.0;
     }
-    gridSum<2>(acc, partial, counter, s);
+#pragma unroll
+    for (int u = 0; u < kDotRows; u++)
+        if ((blockIdx.x * kDotRows + u) * kThreads + (int)threadIdx.x < N) {
+            acc[u][0] = rv[u] * ev[u];
+            if (useQ) acc[u][1] = ev[u] * qv[u];
+        }
+    gridSum<2, kDotRows>(acc, N, partial, counter, s);
 }
 
 // p_new = e + beta p_old (beta = -s[1] / s[pqOld], 0 on the first iteration),
 // q = A p_new, s[pqNew] = (p_new, q). Neighbours' p_new are formed from their
 // e and p_old on the fly, so the direction update needs no pass of its own.
+// WC > 0: the slot count at compile time; every slot's neighbour (from the
+// segment offsets where the mesh has them) and coefficient, then every
+// neighbour's e and p_old, are loaded before the ordered sum.
+template <int WC>
 __global__ void __launch_bounds__(kThreads) k_fcg_spmv(const Ctl* ctl, LevelDev L, const float* __restrict__ e,
                                                        const double* __restrict__ pOld, double* __restrict__ pNew,
                                                        double* __restrict__ q, double* s, int first, int pqOld,
@@ -158,29 +194,72 @@ __global__ void __launch_bounds__(kThreads) k_fcg_spmv(const Ctl* ctl, LevelDev 
                                                        unsigned int* counter) {
     pdlEnter();
     if (ctl->done || ctl->ppSkip) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int G = WC > 0 ? kSpmvRows : 1;
+    constexpr int W = WC > 0 ? WC : 1;
     double beta = 0.0;
     if (!first) {
         const double pq = s[pqOld];
         beta = (pq != 0.0 && isfinite(pq)) ? -s[1] / pq : 0.0;
     }
-    double acc[1] = {0.0};
-    if (n < L.N) {
-        const double pn = first ? (double)e[n] : (double)e[n] + beta * pOld[n];
-        double Ap = L.AC[n] * pn;
-        for (int j = 0; j < L.W; j++) {
-            const size_t sl = (size_t)j * L.N + n;
-            const int k = L.nb[sl];
-            if (k >= 0) {
-                const double pk = first ? (double)e[k] : (double)e[k] + beta * pOld[k];
-                Ap += L.AF[sl] * pk;
+    double acc[G][1] = {};
+    if (WC > 0) {
+        int k[G][W];
+        double a[G][W], ek[G][W], pk[G][W], en[G], po[G], ac[G];
+#pragma unroll
+        for (int u = 0; u < G; u++) {
+            const int n = min((blockIdx.x * G + u) * kThreads + (int)threadIdx.x, L.N - 1);
+            segNeighbours<W>(L.seg, L.nb, L.N, n, k[u]);
+#pragma unroll
+            for (int j = 0; j < W; j++) a[u][j] = L.AF[(size_t)j * L.N + n];
+            en[u] = (double)e[n];
+            po[u] = first ? 0.0 : pOld[n];
+            ac[u] = L.AC[n];
+        }
+#pragma unroll
+        for (int u = 0; u < G; u++) {
+            const int n = min((blockIdx.x * G + u) * kThreads + (int)threadIdx.x, L.N - 1);
+#pragma unroll
+            for (int j = 0; j < W; j++) {
+                const int m = k[u][j] >= 0 ? k[u][j] : n;
+                ek[u][j] = (double)e[m];
+                pk[u][j] = first ? 0.0 : pOld[m];
             }
         }
-        pNew[n] = pn;
-        q[n] = Ap;
-        acc[0] = pn * Ap;
+#pragma unroll
+        for (int u = 0; u < G; u++) {
+            const int n = (blockIdx.x * G + u) * kThreads + (int)threadIdx.x;
+            if (n >= L.N) continue;
+            const double pn = first ? en[u] : en[u] + beta * po[u];
+            double Ap = ac[u] * pn;
+#pragma unroll
+            for (int j = 0; j < W; j++)
+                if (k[u][j] >= 0) {
+                    const double pm = first ? ek[u][j] : ek[u][j] + beta * pk[u][j];
+                    Ap += a[u][j] * pm;
+                }
+            pNew[n] = pn;
+            q[n] = Ap;
+            acc[u][0] = pn * Ap;
+        }
+    } else {
+        const int n = blockIdx.x * blockDim.x + threadIdx.x;
+        if (n < L.N) {
+            const double pn = first ? (double)e[n] : (double)e[n] + beta * pOld[n];
+            double Ap = L.AC[n] * pn;
+            for (int j = 0; j < L.W; j++) {
+                const size_t sl = (size_t)j * L.N + n;
+                const int k = L.nb[sl];
+                if (k >= 0) {
+                    const double pk = first ? (double)e[k] : (double)e[k] + beta * pOld[k];
+                    Ap += L.AF[sl] * pk;
+                }
+            }
+            pNew[n] = pn;
+            q[n] = Ap;
+            acc[0][0] = pn * Ap;
+        }
     }
-    gridSum<1>(acc, partial, counter, s + pqNew);
+    gridSum<1, G>(acc, L.N, partial, counter, s + pqNew);
 }
 
 // alpha = s[0] / s[pq]; x += alpha p; r -= alpha q; r in FP32 (and the first
@@ -193,31 +272,41 @@ __global__ void __launch_bounds__(kThreads) k_fcg_update(Ctl* ctl, LevelDev L, d
                                                          double* __restrict__ partial, unsigned int* counter) {
     pdlEnter();
     if (ctl->done || ctl->ppSkip) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int G = kUpdateRows;
     const double pq = s[pqSlot];
     const double alpha = (pq != 0.0 && isfinite(pq)) ? s[0] / pq : 0.0;
-    double acc[1] = {0.0};
-    if (n < L.N) {
-        x[n] += alpha * p[n];
+    double acc[G][1] = {};
+    double xv[G], pv[G], rv[G], qv[G], ac[G];
+#pragma unroll
+    for (int u = 0; u < G; u++) {
+        const int n = min((blockIdx.x * G + u) * kThreads + (int)threadIdx.x, L.N - 1);
+        xv[u] = x[n];
+        pv[u] = p[n];
+        rv[u] = next ? r[n] : 0.0;
+        qv[u] = next ? q[n] : 0.0;
+        ac[u] = next > 1 ? L.AC[n] : 1.0;
+    }
+#pragma unroll
+    for (int u = 0; u < G; u++) {
+        const int n = (blockIdx.x * G + u) * kThreads + (int)threadIdx.x;
+        if (n >= L.N) continue;
+        x[n] = xv[u] + alpha * pv[u];
         if (next) {
-            const double rv = r[n] - alpha * q[n];
-            r[n] = rv;
-            r32[n] = (float)rv;
-            if (next > 1) {
-                const double ac = L.AC[n];
-                eFirst[n] = (fabs(ac) < 1.0e-30) ? 0.f : (float)(w * rv / ac);
-            }
-            acc[0] = rv * rv;
+            const double rn = rv[u] - alpha * qv[u];
+            r[n] = rn;
+            r32[n] = (float)rn;
+            if (next > 1) eFirst[n] = (fabs(ac[u]) < 1.0e-30) ? 0.f : (float)(w * rn / ac[u]);
+            acc[u][0] = rn * rn;
         }
     }
     if (!next) {
-        if (n == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
             ctl->ppIterations++;
             if (ctl->ppIterations - (long long)s[6] >= maxIt) ctl->ppSkip = 1;
         }
         return;
     }
-    if (gridSum<1>(acc, partial, counter, s + 5)) {
+    if (gridSum<1, G>(acc, L.N, partial, counter, s + 5)) {
         ctl->ppIterations++;
         if (s[5] <= relTol * relTol * s[4] || ctl->ppIterations - (long long)s[6] >= maxIt) ctl->ppSkip = 1;
     }
@@ -264,7 +353,7 @@ __global__ void __launch_bounds__(kThreads) k_nn_scale(const Ctl* ctl, LevelDev 
     pdlEnter();
     if (ctl->done || ctl->ppSkip != 2) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    double acc[2] = {0.0, 0.0};
+    double acc[1][2] = {};
     if (n < L.N) {
         const double yn = (double)y[n];
         double a = L.AC[n] * yn;
@@ -274,10 +363,10 @@ __global__ void __launch_bounds__(kThreads) k_nn_scale(const Ctl* ctl, LevelDev 
             if (k >= 0) a += L.AF[s] * (double)y[k];
         }
         Ay[n] = a;
-        acc[0] = yn * r[n];
-        acc[1] = yn * a;
+        acc[0][0] = yn * r[n];
+        acc[0][1] = yn * a;
     }
-    if (gridSum<2>(acc, partial, counter, sn + 1)) sn[0] = (sn[2] > 0.0 && isfinite(sn[1])) ? sn[1] / sn[2] : 0.0;
+    if (gridSum<2, 1>(acc, L.N, partial, counter, sn + 1)) sn[0] = (sn[2] > 0.0 && isfinite(sn[1])) ? sn[1] / sn[2] : 0.0;
 }
 
 // Step 2: r' = r - alpha A y in FP64, r' in FP32 for the V-cycle that follows,
@@ -344,20 +433,28 @@ void launchFcgInit(Ctl* ctl, const LevelDev& L0, const double* x, double* r, flo
 
 void launchFcgDots(const Ctl* ctl, int N, const float* e, const double* r, const double* q, int useQ, FcgScratch& f,
                    cudaStream_t s) {
-    launchPDL(k_fcg_dots, dim3(blocksFor(N)), dim3(kThreads), 0, s, ctl, N, e, r, q, useQ, f.partial, f.counter,
+    launchPDL(k_fcg_dots, dim3(blocksFor(N, kDotRows)), dim3(kThreads), 0, s, ctl, N, e, r, q, useQ, f.partial, f.counter,
               f.scalars);
 }
 
 void launchFcgSpmv(const Ctl* ctl, const LevelDev& L0, const float* e, const double* pOld, double* pNew, double* q,
                    int first, int pqOld, int pqNew, FcgScratch& f, cudaStream_t s) {
-    launchPDL(k_fcg_spmv, dim3(blocksFor(L0.N)), dim3(kThreads), 0, s, ctl, L0, e, pOld, pNew, q, f.scalars, first,
-              pqOld, pqNew, f.partial, f.counter + 1);
+    const dim3 grid(blocksFor(L0.N, L0.W == 3 || L0.W == 4 ? kSpmvRows : 1));
+    if (L0.W == 4)
+        launchPDL(k_fcg_spmv<4>, grid, dim3(kThreads), 0, s, ctl, L0, e, pOld, pNew, q, f.scalars, first, pqOld, pqNew,
+                  f.partial, f.counter + 1);
+    else if (L0.W == 3)
+        launchPDL(k_fcg_spmv<3>, grid, dim3(kThreads), 0, s, ctl, L0, e, pOld, pNew, q, f.scalars, first, pqOld, pqNew,
+                  f.partial, f.counter + 1);
+    else
+        launchPDL(k_fcg_spmv<0>, grid, dim3(kThreads), 0, s, ctl, L0, e, pOld, pNew, q, f.scalars, first, pqOld, pqNew,
+                  f.partial, f.counter + 1);
 }
 
 void launchFcgUpdate(Ctl* ctl, const LevelDev& L0, double* x, double* r, const double* p, const double* q,
                      FcgScratch& f, int pqSlot, float* r32, float* eFirst, double w, int next, double relTol,
                      int maxIt, cudaStream_t s) {
-    launchPDL(k_fcg_update, dim3(blocksFor(L0.N)), dim3(kThreads), 0, s, ctl, L0, x, r, p, q, f.scalars, pqSlot, r32,
+    launchPDL(k_fcg_update, dim3(blocksFor(L0.N, kUpdateRows)), dim3(kThreads), 0, s, ctl, L0, x, r, p, q, f.scalars, pqSlot, r32,
               eFirst, w, next, relTol, maxIt, f.partial, f.counter + 1);
 }
 
