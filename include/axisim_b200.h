@@ -486,6 +486,7 @@ int axisim_mesh_segments(axisim_handle* h, int32_t* nSegments, int32_t* nOffsetS
  * allocation: for callers that cannot allocate at that point -- a host whose
  * GPU memory is all held by another allocator or capped, or a monitoring hook
  * inside a time-critical loop where cudaMalloc/cudaFree would stall the device.
+ * The first call of a process page-locks 16 KB of host memory for the status.
  * The reduction scratch is a fixed file-scope device array sized for at most
  * AXISIM_STATIC_MAX_CELLS cells; larger nCells is rejected with AXISIM_E_ARG.
  * Inputs, all device pointers on the current device, in the reference's CSR
