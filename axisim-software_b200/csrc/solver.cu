@@ -1578,11 +1578,14 @@ private:
     ResidentArgsT<float>* rec32_ = nullptr;
     double recBytes_ = 0.0;
     int residentVcycle_ = 0;
-    // coarse levels up to this size fuse residual + restriction and
-    // prolongation + first post-sweep (beyond it the fused forms, one thread
-    // per row gathering its neighbours' corrections, run slower than two
-    // coalesced passes)
+    // coarse levels up to this size fuse the prolongation and the first
+    // post-sweep (beyond it the fused form, one thread per row gathering its
+    // neighbours' corrections, runs slower than two coalesced passes)
     static constexpr int kFuseMaxCells = 65536;
+    // the restriction with residual (four lanes a coarse cell) up to this size:
+    // against 65,536, 2M cells FCG 23.65 -> 23.41 ms, bullet 7.32 -> 7.25, 874k FP64
+    // 9.10 -> 9.05, mixed equal (15.48)
+    static constexpr int kFuseGatherCells = 262144;
     int barrierPhantom_ = 0;  // test hook: extra arrivals each grid barrier expects
     bool timedOut_ = false;   // the last run ended on a barrier that gave up
     template <class T>
@@ -1638,7 +1641,7 @@ private:
         // levels, the finest one (coalesced [W][N] rows) and the level above
         // the tail (whose residual the tail reads) keep the separate pass
         const bool tail = l + 1 == tailStart_ && (l + 1 != cluster_.first || residentVcycle_);
-        const bool gatherRes = F.sliceOff != nullptr && F.N <= kFuseMaxCells && !tail;
+        const bool gatherRes = F.sliceOff != nullptr && F.N <= kFuseGatherCells && !tail;
         if (!gatherRes) {
             T* x = cur[(size_t)l];
             emit<T>(kOpResidual, l, x, nullptr, 0, 0.0, 0, std::string("mg_residual") + tag,
