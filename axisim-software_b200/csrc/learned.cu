@@ -130,6 +130,7 @@ __device__ bool gridSumD(const double (&v)[NQ], double* partial, unsigned int* c
 template <class TR>
 __global__ void __launch_bounds__(kThreads) k_sigma(const Ctl* ctl, int gated, int N, const TR* r, const TR* AC, double* partial,
                                                     unsigned int* counter, double* scal) {
+    pdlEnter();
     if (idle(ctl, gated)) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[1] = {0.0};
@@ -147,6 +148,7 @@ template <class TA, class TR>
 __global__ void __launch_bounds__(kThreads) k_features(const Ctl* ctl, int gated, int N, const TR* r, const TR* AC,
                                                        const double* AF, const int32_t* nb, int W,
                                                        const float* deficit, const double* scal, TA* feat) {
+    pdlEnter();
     if (idle(ctl, gated)) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N) return;
@@ -194,6 +196,7 @@ __device__ __forceinline__ void gatherInput(const NetIn& I, int n, float* z) {
 // (stride K + 1: conflict-free across the warp), weights are broadcast loads.
 template <class TA, class TW, int OCH>
 __global__ void k_layer_fwd(const Ctl* ctl, int gated, NetLayer L, const TW* __restrict__ P) {
+    pdlEnter();
     if (idle(ctl, gated)) return;
     extern __shared__ float zsm[];
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -296,6 +299,7 @@ __device__ __forceinline__ void gatherTile(const NetLayer& L, int row0, float* z
 
 template <class TA, class TW, int CPT, int RPT>
 __global__ void __launch_bounds__(256) k_layer_tile(const Ctl* ctl, int gated, NetLayer L, const TW* __restrict__ P) {
+    pdlEnter();
     if (idle(ctl, gated)) return;
     constexpr int COUT = 16 * CPT;
     constexpr int TR = 16 * RPT;  // rows per tile
@@ -409,6 +413,7 @@ __global__ void __launch_bounds__(256) k_layer_tile(const Ctl* ctl, int gated, N
 template <class TA, class TW, int KPT>
 __global__ void __launch_bounds__(256) k_layer_dz_tile(NetLayer L, const TW* __restrict__ P, float* __restrict__ G,
                                                        float* __restrict__ dZ) {
+    pdlEnter();
     constexpr int KD = 16 * KPT;
     extern __shared__ float sm[];
     const int Cout = L.Cout;
@@ -576,6 +581,7 @@ struct PackArgs {
 };
 __global__ void __launch_bounds__(kThreads) k_pack(PackArgs a, const bfloat* __restrict__ low, bfloat* __restrict__ fwd,
                                                    bfloat* __restrict__ bwd) {
+    pdlEnter();
     const unsigned int off = a.off[blockIdx.y];
     const int K = a.K[blockIdx.y], Cout = a.Cout[blockIdx.y];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < K * Cout; i += gridDim.x * blockDim.x) {
@@ -642,6 +648,7 @@ template <class TA, int NB>
 __global__ void __launch_bounds__(kMmaThreads) k_layer_mma(const Ctl* ctl, int gated, NetLayer L,
                                                            const bfloat* __restrict__ P,
                                                            const bfloat* __restrict__ packed) {
+    pdlEnter();
     if (idle(ctl, gated)) return;
     extern __shared__ __align__(16) uint2 wsm[];
     const int K = L.K, Cout = L.Cout;
@@ -739,6 +746,7 @@ __global__ void __launch_bounds__(kMmaThreads) k_layer_mma(const Ctl* ctl, int g
 template <class TA, int NB>
 __global__ void __launch_bounds__(kMmaThreads) k_layer_dz_mma(NetLayer L, const bfloat* __restrict__ packed,
                                                               float* __restrict__ G, float* __restrict__ dZ) {
+    pdlEnter();
     extern __shared__ __align__(16) uint2 wsm[];
     const int K = L.K, Cout = L.Cout;
     stageWeights(wsm, packed + L.wOff, Cout, K);
@@ -791,6 +799,7 @@ __global__ void __launch_bounds__(kMmaThreads) k_layer_dz_mma(NetLayer L, const 
 template <class TA>
 __global__ void __launch_bounds__(kThreads) k_layer_in(const Ctl* ctl, int gated, NetLayer L,
                                                        const bfloat* __restrict__ P) {
+    pdlEnter();
     if (idle(ctl, gated)) return;
     const int per = L.Cout / 4;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -810,6 +819,7 @@ __global__ void __launch_bounds__(kThreads) k_layer_in(const Ctl* ctl, int gated
 template <class TA>
 __global__ void __launch_bounds__(kThreads) k_layer_out(const Ctl* ctl, int gated, NetLayer L,
                                                         const bfloat* __restrict__ P) {
+    pdlEnter();
     if (idle(ctl, gated)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = i >> 2, t4 = i & 3;
@@ -823,6 +833,7 @@ __global__ void __launch_bounds__(kThreads) k_layer_out(const Ctl* ctl, int gate
 
 // Its input gradient straight into the source's: gX[n][k] += g[n] w[k].
 __global__ void __launch_bounds__(kThreads) k_adj_out(NetLayer L, const bfloat* __restrict__ P, float* __restrict__ gX) {
+    pdlEnter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = i >> 2, t4 = i & 3;
     if (n >= L.N) return;
@@ -838,6 +849,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_out(NetLayer L, const bfloat* 
 template <class TA>
 __global__ void __launch_bounds__(kThreads) k_mask(size_t n4, const float* __restrict__ gY, const TA* __restrict__ Y,
                                                    float* __restrict__ G) {
+    pdlEnter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n4) return;
     float4 v = ldv4(gY + 4 * i);
@@ -853,6 +865,7 @@ __global__ void __launch_bounds__(kThreads) k_mask(size_t n4, const float* __res
 template <class TA>
 __global__ void __launch_bounds__(kThreads) k_scale_out(const Ctl* ctl, int gated, int N, const TA* y, const double* scal,
                                                         float* e) {
+    pdlEnter();
     if (idle(ctl, gated)) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N) return;
@@ -871,6 +884,7 @@ __global__ void __launch_bounds__(kThreads) k_loss_spmv(int N, int W, const int3
                                                         const float* __restrict__ AF, const float* __restrict__ AC,
                                                         const TA* y, const float* b, const float* t, float* Ay,
                                                         double* partial, unsigned int* counter, double* scal) {
+    pdlEnter();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[3] = {0.0, 0.0, 0.0};
     if (n < N) {
@@ -893,6 +907,7 @@ __global__ void __launch_bounds__(kThreads) k_loss_spmv(int N, int W, const int3
 // E_y = y.Ay, E_t = b.t (A symmetric)
 __global__ void __launch_bounds__(kThreads) k_loss_grad(int N, const float* b, const float* Ay, const double* scal,
                                                         float* gy, float* lossOut) {
+    pdlEnter();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const double c = scal[1], ey = scal[2] > 0.0 ? scal[2] : 1e-300, et = scal[3] > 0.0 ? scal[3] : 1.0;
     if (n == 0) *lossOut = (float)(1.0 - c * c / (ey * et));
@@ -906,6 +921,7 @@ __global__ void __launch_bounds__(kThreads) k_loss_grad(int N, const float* b, c
 template <class TA, class TW, int KCH>
 __global__ void __launch_bounds__(kThreads) k_layer_dz(NetLayer L, const TW* __restrict__ P, float* __restrict__ G,
                                                        float* __restrict__ dZ) {
+    pdlEnter();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= L.N) return;
     const int K = L.K, Cout = L.Cout;
@@ -940,6 +956,7 @@ template <class TA>
 __global__ void __launch_bounds__(kThreads) k_wgrad(int N, int K, int Cout, int tilesO, int rowsPerSplit,
                                                     const TA* __restrict__ Z, const float* __restrict__ G,
                                                     float* __restrict__ partial) {
+    pdlEnter();
     __shared__ float zs[64][33];
     __shared__ float gs[64][33];
     const int tk = blockIdx.x / tilesO, to = blockIdx.x % tilesO;
@@ -1017,6 +1034,7 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(int N, int K, int Cout, int 
 // grad += the sum of the splits: 32 entries a block, eight threads an entry
 __global__ void __launch_bounds__(kThreads) k_wgrad_reduce(int entries, int splits, const float* __restrict__ partial,
                                                            float* __restrict__ grad) {
+    pdlEnter();
     __shared__ float sh[8][32];
     const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
     const int e = blockIdx.x * 32 + lane;
@@ -1044,6 +1062,7 @@ __device__ __forceinline__ float4 scaled(float4 v, float w) { return make_float4
 
 __global__ void __launch_bounds__(kThreads) k_adj_id(int N, int C, int off, int K, const float* __restrict__ dZ,
                                                      float* __restrict__ gX) {
+    pdlEnter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)C / 4;
     if (i >= (size_t)N * per) return;
     accumulate4(gX + 4 * i, ldv4(dZ + (i / per) * K + off + 4 * (i % per)));
@@ -1054,6 +1073,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_id(int N, int C, int off, int 
 __global__ void __launch_bounds__(kThreads) k_adj_mp(int N, int C, int K, const int32_t* __restrict__ s,
                                                      const int32_t* __restrict__ list, const float* __restrict__ inv,
                                                      const float* __restrict__ dZ, float* __restrict__ gX) {
+    pdlEnter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)C / 4;
     if (i >= (size_t)N * per) return;
     const int k = (int)(i / per), c = (int)(i % per) * 4;
@@ -1090,6 +1110,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_mp(int N, int C, int K, const 
 __global__ void __launch_bounds__(kThreads) k_adj_pool(int Nf, int C, int off, int K, const int32_t* __restrict__ c2c,
                                                        const float* __restrict__ invCnt, const float* __restrict__ dZ,
                                                        float* __restrict__ gX) {
+    pdlEnter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)C / 4;
     if (i >= (size_t)Nf * per) return;
     const int cc = c2c[i / per];
@@ -1100,6 +1121,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_pool(int Nf, int C, int off, i
 __global__ void __launch_bounds__(kThreads) k_adj_unpool(int Nc, int C, int off, int K, const int32_t* __restrict__ ms,
                                                          const int32_t* __restrict__ ml, const float* __restrict__ dZ,
                                                          float* __restrict__ gX) {
+    pdlEnter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)C / 4;
     if (i >= (size_t)Nc * per) return;
     const int c = (int)(i / per);
@@ -1114,6 +1136,7 @@ template <class TW>
 __global__ void __launch_bounds__(kThreads) k_adam(size_t n, float* __restrict__ p, const float* __restrict__ g,
                                                    float* __restrict__ m, float* __restrict__ v, TW* low, float lr,
                                                    float b1, float b2, float eps, float c1, float c2) {
+    pdlEnter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -1128,6 +1151,7 @@ __global__ void __launch_bounds__(kThreads) k_adam(size_t n, float* __restrict__
 
 template <class TW>
 __global__ void __launch_bounds__(kThreads) k_to_low(size_t n, const float* __restrict__ p, TW* __restrict__ low) {
+    pdlEnter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) stv(low, i, p[i]);
 }
@@ -1140,6 +1164,7 @@ __global__ void __launch_bounds__(kThreads) k_harvest(const Ctl* ctl, int N, int
                                                       const double* x, const double* AC, const double* AF,
                                                       const int32_t* nb, int W, const double* fs, float* store,
                                                       int* count, float* relres, unsigned int* counter) {
+    pdlEnter();
     if (ctl->done || every <= 0 || (ctl->currentIteration % every) != 0) return;
     const int slot = *(volatile int*)count;
     if (slot >= cap) return;
@@ -1195,7 +1220,7 @@ void launchTileR(const Ctl* ctl, int gated, const NetLayer& L, const void* P, cu
     const size_t smem =
         ((size_t)16 * RPT * (L.K + 1) + (size_t)kChunk * 16 * CPT + 16 * RPT + 1) * sizeof(float);
     allowSmem(k_layer_tile<TA, TW, CPT, RPT>, smem);
-    k_layer_tile<TA, TW, CPT, RPT><<<blocksFor(L.N, 16 * RPT), 256, smem, s>>>(ctl, gated, L, (const TW*)P);
+    launchPDL(k_layer_tile<TA, TW, CPT, RPT>, dim3(blocksFor(L.N, 16 * RPT)), dim3(256), smem, s, ctl, gated, L, (const TW*)P);
 }
 
 // 64-row tiles on large levels; 16-row tiles (4 x the blocks, 1/4 the work
@@ -1210,7 +1235,7 @@ template <class TA, class TW, int KPT>
 void launchDzTile(const NetLayer& L, const void* P, float* G, float* dZ, cudaStream_t s) {
     const size_t smem = ((size_t)kTileRows * (L.Cout + 1) + (size_t)kChunk * 16 * KPT) * sizeof(float);
     allowSmem(k_layer_dz_tile<TA, TW, KPT>, smem);
-    k_layer_dz_tile<TA, TW, KPT><<<blocksFor(L.N, kTileRows), 256, smem, s>>>(L, (const TW*)P, G, dZ);
+    launchPDL(k_layer_dz_tile<TA, TW, KPT>, dim3(blocksFor(L.N, kTileRows)), dim3(256), smem, s, L, (const TW*)P, G, dZ);
 }
 
 // The tiled kernels assume every channel count divides their 256 threads.
@@ -1246,7 +1271,7 @@ void launchMmaNB(const Ctl* ctl, int gated, const NetLayer& L, const bfloat* P, 
     const size_t smem = (size_t)L.K * L.Cout * sizeof(bfloat);
     allowSmem(k_layer_mma<TA, NB>, smem);
     const int perCta = (kMmaThreads / 32) / (L.Cout / (8 * NB));
-    k_layer_mma<TA, NB><<<mmaCtas(L, perCta, smem), kMmaThreads, smem, s>>>(ctl, gated, L, P, packed);
+    launchPDL(k_layer_mma<TA, NB>, dim3(mmaCtas(L, perCta, smem)), dim3(kMmaThreads), smem, s, ctl, gated, L, P, packed);
 }
 template <class TA>
 void launchMma(const Ctl* ctl, int gated, const NetLayer& L, const bfloat* P, const bfloat* packed, cudaStream_t s) {
@@ -1261,7 +1286,7 @@ void launchDzMmaNB(const NetLayer& L, const bfloat* packed, float* G, float* dZ,
     const size_t smem = (size_t)L.K * L.Cout * sizeof(bfloat);
     allowSmem(k_layer_dz_mma<TA, NB>, smem);
     const int perCta = (kMmaThreads / 32) / (L.K / (8 * NB));
-    k_layer_dz_mma<TA, NB><<<mmaCtas(L, perCta, smem), kMmaThreads, smem, s>>>(L, packed, G, dZ);
+    launchPDL(k_layer_dz_mma<TA, NB>, dim3(mmaCtas(L, perCta, smem)), dim3(kMmaThreads), smem, s, L, packed, G, dZ);
 }
 template <class TA>
 void launchDzMma(const NetLayer& L, const bfloat* packed, float* G, float* dZ, cudaStream_t s) {
@@ -1277,8 +1302,8 @@ template <class TA>
 void launchLayerLow(const Ctl* ctl, int gated, const NetLayer& L, const bfloat* P, const bfloat* packed,
                     cudaStream_t s) {
     if (slabs(L)) launchMma<TA>(ctl, gated, L, P, packed, s);
-    else if (L.K == 2) k_layer_in<TA><<<blocksFor((size_t)L.N * L.Cout / 4), kThreads, 0, s>>>(ctl, gated, L, P);
-    else k_layer_out<TA><<<blocksFor((size_t)L.N * 4), kThreads, 0, s>>>(ctl, gated, L, P);
+    else if (L.K == 2) launchPDL(k_layer_in<TA>, dim3(blocksFor((size_t)L.N * L.Cout / 4)), dim3(kThreads), 0, s, ctl, gated, L, P);
+    else launchPDL(k_layer_out<TA>, dim3(blocksFor((size_t)L.N * 4)), dim3(kThreads), 0, s, ctl, gated, L, P);
 }
 
 template <class TA, class TW>
@@ -1294,9 +1319,9 @@ void launchLayerFwd(const Ctl* ctl, int gated, const NetLayer& L, const void* P,
     const size_t smem = (size_t)rows * (L.K + 1) * sizeof(float);
     const dim3 grid(blocksFor(L.N, rows));
     const TW* p = (const TW*)P;
-    if (L.Cout >= 32) k_layer_fwd<TA, TW, 32><<<grid, rows, smem, s>>>(ctl, gated, L, p);
-    else if (L.Cout >= 16) k_layer_fwd<TA, TW, 16><<<grid, rows, smem, s>>>(ctl, gated, L, p);
-    else k_layer_fwd<TA, TW, 1><<<grid, rows, smem, s>>>(ctl, gated, L, p);
+    if (L.Cout >= 32) launchPDL(k_layer_fwd<TA, TW, 32>, dim3(grid), dim3(rows), smem, s, ctl, gated, L, p);
+    else if (L.Cout >= 16) launchPDL(k_layer_fwd<TA, TW, 16>, dim3(grid), dim3(rows), smem, s, ctl, gated, L, p);
+    else launchPDL(k_layer_fwd<TA, TW, 1>, dim3(grid), dim3(rows), smem, s, ctl, gated, L, p);
 }
 
 template <class TA, class TW>
@@ -1311,7 +1336,7 @@ void launchLayerDz(const NetLayer& L, const void* P, float* G, float* dZ, cudaSt
             default: break;
         }
     }
-    k_layer_dz<TA, TW, 16><<<blocksFor(L.N), kThreads, 0, s>>>(L, (const TW*)P, G, dZ);
+    launchPDL(k_layer_dz<TA, TW, 16>, dim3(blocksFor(L.N)), dim3(kThreads), 0, s, L, (const TW*)P, G, dZ);
 }
 
 template <class T>
@@ -1342,7 +1367,7 @@ inline int wgradSplits(const NetLayer& L) {
 void launchHarvest(const Ctl* ctl, int N, int every, int cap, const double* b, const double* x, const double* AC,
                    const double* AF, const int32_t* nb, int W, const double* fcgScalars, float* store, int* count,
                    float* relres, unsigned int* counter, cudaStream_t s) {
-    k_harvest<<<blocksFor(N), kThreads, 0, s>>>(ctl, N, every, cap, b, x, AC, AF, nb, W, fcgScalars, store, count,
+    launchPDL(k_harvest, dim3(blocksFor(N)), dim3(kThreads), 0, s, ctl, N, every, cap, b, x, AC, AF, nb, W, fcgScalars, store, count,
                                                 relres, counter);
 }
 
@@ -1609,7 +1634,7 @@ void LearnedNet::buildLayers() {
 
 void LearnedNet::syncLowPrecision(cudaStream_t s) {
     if (!wBf16_) return;
-    k_to_low<bfloat><<<blocksFor(nParams_), kThreads, 0, s>>>(nParams_, params_, (bfloat*)paramsLow_);
+    launchPDL(k_to_low<bfloat>, dim3(blocksFor(nParams_)), dim3(kThreads), 0, s, nParams_, params_, (bfloat*)paramsLow_);
     packWeights(s);
     NCK(cudaGetLastError());
 }
@@ -1629,7 +1654,7 @@ void LearnedNet::packWeights(cudaStream_t s) {
         a.Cout[a.n] = (short)L.Cout;
         a.n++;
     }
-    if (a.n) k_pack<<<dim3(16, a.n), kThreads, 0, s>>>(a, (const bfloat*)paramsLow_, (bfloat*)packF_, (bfloat*)packB_);
+    if (a.n) launchPDL(k_pack, dim3(dim3(16, a.n)), dim3(kThreads), 0, s, a, (const bfloat*)paramsLow_, (bfloat*)packF_, (bfloat*)packB_);
 }
 
 void LearnedNet::forward(const Ctl* ctl, int gated, bool keepZ, cudaStream_t s) {
@@ -1644,16 +1669,16 @@ void LearnedNet::forward(const Ctl* ctl, int gated, bool keepZ, cudaStream_t s) 
 void LearnedNet::infer(const Ctl* ctl, int gated, const double* r, const double* AC, const double* AF,
                        const int32_t* nb, int W, float* e, cudaStream_t s) {
     const int nb0 = blocksFor(N0_);
-    k_sigma<double><<<nb0, kThreads, 0, s>>>(ctl, gated, N0_, r, AC, red_, counter_, scal_);
+    launchPDL(k_sigma<double>, dim3(nb0), dim3(kThreads), 0, s, ctl, gated, N0_, r, AC, red_, counter_, scal_);
     if (actBf16_)
-        k_features<bfloat, double><<<nb0, kThreads, 0, s>>>(ctl, gated, N0_, r, AC, AF, nb, W, nullptr, scal_,
+        launchPDL(k_features<bfloat, double>, dim3(nb0), dim3(kThreads), 0, s, ctl, gated, N0_, r, AC, AF, nb, W, nullptr, scal_,
                                                              (bfloat*)feat_);
     else
-        k_features<float, double><<<nb0, kThreads, 0, s>>>(ctl, gated, N0_, r, AC, AF, nb, W, nullptr, scal_,
+        launchPDL(k_features<float, double>, dim3(nb0), dim3(kThreads), 0, s, ctl, gated, N0_, r, AC, AF, nb, W, nullptr, scal_,
                                                             (float*)feat_);
     forward(ctl, gated, false, s);
-    if (actBf16_) k_scale_out<bfloat><<<nb0, kThreads, 0, s>>>(ctl, gated, N0_, (const bfloat*)out_, scal_, e);
-    else k_scale_out<float><<<nb0, kThreads, 0, s>>>(ctl, gated, N0_, (const float*)out_, scal_, e);
+    if (actBf16_) launchPDL(k_scale_out<bfloat>, dim3(nb0), dim3(kThreads), 0, s, ctl, gated, N0_, (const bfloat*)out_, scal_, e);
+    else launchPDL(k_scale_out<float>, dim3(nb0), dim3(kThreads), 0, s, ctl, gated, N0_, (const float*)out_, scal_, e);
 }
 
 void LearnedNet::backward(cudaStream_t s) {
@@ -1666,11 +1691,11 @@ void LearnedNet::backward(cudaStream_t s) {
             launchLayerDz<float, float>(L, paramsLow_, gpre_, needDz ? dZ_ : nullptr, s);
         } else if (direct) {
             G = L.gY;
-            k_adj_out<<<blocksFor((size_t)L.N * 4), kThreads, 0, s>>>(L, (const bfloat*)paramsLow_, L.gIn[0]);
+            launchPDL(k_adj_out, dim3(blocksFor((size_t)L.N * 4)), dim3(kThreads), 0, s, L, (const bfloat*)paramsLow_, L.gIn[0]);
         } else if (!needDz) {
             const size_t n4 = (size_t)L.N * L.Cout / 4;
-            if (actBf16_) k_mask<bfloat><<<blocksFor(n4), kThreads, 0, s>>>(n4, L.gY, (const bfloat*)L.Y, gpre_);
-            else k_mask<float><<<blocksFor(n4), kThreads, 0, s>>>(n4, L.gY, (const float*)L.Y, gpre_);
+            if (actBf16_) launchPDL(k_mask<bfloat>, dim3(blocksFor(n4)), dim3(kThreads), 0, s, n4, L.gY, (const bfloat*)L.Y, gpre_);
+            else launchPDL(k_mask<float>, dim3(blocksFor(n4)), dim3(kThreads), 0, s, n4, L.gY, (const float*)L.Y, gpre_);
         } else if (actBf16_) {
             launchDzMma<bfloat>(L, (const bfloat*)packB_, gpre_, dZ_, s);
         } else {
@@ -1683,18 +1708,18 @@ void LearnedNet::backward(cudaStream_t s) {
         const int tilesK = (L.K + 31) / 32, tilesO = (L.Cout + 31) / 32;
         const dim3 grid((unsigned)(tilesK * tilesO), (unsigned)splits);
         if (actBf16_)
-            k_wgrad<bfloat><<<grid, kThreads, 0, s>>>(L.N, L.K, L.Cout, tilesO, rowsPerSplit, (const bfloat*)Z, G,
+            launchPDL(k_wgrad<bfloat>, dim3(grid), dim3(kThreads), 0, s, L.N, L.K, L.Cout, tilesO, rowsPerSplit, (const bfloat*)Z, G,
                                                       wgPartial_);
         else
-            k_wgrad<float><<<grid, kThreads, 0, s>>>(L.N, L.K, L.Cout, tilesO, rowsPerSplit, (const float*)Z, G,
+            launchPDL(k_wgrad<float>, dim3(grid), dim3(kThreads), 0, s, L.N, L.K, L.Cout, tilesO, rowsPerSplit, (const float*)Z, G,
                                                      wgPartial_);
         const int entries = L.K * L.Cout + L.Cout;
-        k_wgrad_reduce<<<blocksFor(entries, 32), kThreads, 0, s>>>(entries, splits, wgPartial_, grad_ + L.wOff);
+        launchPDL(k_wgrad_reduce, dim3(blocksFor(entries, 32)), dim3(kThreads), 0, s, entries, splits, wgPartial_, grad_ + L.wOff);
         // adjoints of the inputs
         int off = 0;
         if (L.nIn == 2) {  // message passing: both inputs are the same tensor
             const NetIn& I = L.in[1];
-            k_adj_mp<<<blocksFor((size_t)L.N * I.C / 4), kThreads, 0, s>>>(L.N, I.C, L.K, I.s, I.list, I.inv, dZ_,
+            launchPDL(k_adj_mp, dim3(blocksFor((size_t)L.N * I.C / 4)), dim3(kThreads), 0, s, L.N, I.C, L.K, I.s, I.list, I.inv, dZ_,
                                                                          L.gIn[1]);
         }
         for (int q = 0; q < L.nIn && L.nIn == 1 && !direct; q++) {
@@ -1704,13 +1729,13 @@ void LearnedNet::backward(cudaStream_t s) {
                 const size_t n = (size_t)I.srcRows * I.C / 4;
                 switch (I.xf) {
                     case NX_ID:
-                        k_adj_id<<<blocksFor(n), kThreads, 0, s>>>(I.srcRows, I.C, off, L.K, dZ_, gX);
+                        launchPDL(k_adj_id, dim3(blocksFor(n)), dim3(kThreads), 0, s, I.srcRows, I.C, off, L.K, dZ_, gX);
                         break;
                     case NX_POOL:
-                        k_adj_pool<<<blocksFor(n), kThreads, 0, s>>>(I.srcRows, I.C, off, L.K, I.map, I.inv, dZ_, gX);
+                        launchPDL(k_adj_pool, dim3(blocksFor(n)), dim3(kThreads), 0, s, I.srcRows, I.C, off, L.K, I.map, I.inv, dZ_, gX);
                         break;
                     default:
-                        k_adj_unpool<<<blocksFor(n), kThreads, 0, s>>>(I.srcRows, I.C, off, L.K, I.s, I.list, dZ_, gX);
+                        launchPDL(k_adj_unpool, dim3(blocksFor(n)), dim3(kThreads), 0, s, I.srcRows, I.C, off, L.K, I.s, I.list, dZ_, gX);
                         break;
                 }
             }
@@ -1718,7 +1743,7 @@ void LearnedNet::backward(cudaStream_t s) {
         }
         if (L.gAdd) {
             const size_t n = (size_t)L.N * L.Cout / 4;
-            k_adj_id<<<blocksFor(n), kThreads, 0, s>>>(L.N, L.Cout, 0, L.Cout, gpre_, L.gAdd);
+            launchPDL(k_adj_id, dim3(blocksFor(n)), dim3(kThreads), 0, s, L.N, L.Cout, 0, L.Cout, gpre_, L.gAdd);
         }
     }
     NCK(cudaGetLastError());
@@ -1726,21 +1751,21 @@ void LearnedNet::backward(cudaStream_t s) {
 
 void LearnedNet::lossAndGrad(const Sample& smp, float* lossOut, cudaStream_t s) {
     const int nb0 = blocksFor(N0_);
-    k_sigma<float><<<nb0, kThreads, 0, s>>>(nullptr, 0, N0_, smp.b, smp.AC, red_, counter_, scal_);
+    launchPDL(k_sigma<float>, dim3(nb0), dim3(kThreads), 0, s, nullptr, 0, N0_, smp.b, smp.AC, red_, counter_, scal_);
     if (actBf16_)
-        k_features<bfloat, float><<<nb0, kThreads, 0, s>>>(nullptr, 0, N0_, smp.b, smp.AC, nullptr, nullptr, 0,
+        launchPDL(k_features<bfloat, float>, dim3(nb0), dim3(kThreads), 0, s, nullptr, 0, N0_, smp.b, smp.AC, nullptr, nullptr, 0,
                                                            smp.deficit, scal_, (bfloat*)feat_);
     else
-        k_features<float, float><<<nb0, kThreads, 0, s>>>(nullptr, 0, N0_, smp.b, smp.AC, nullptr, nullptr, 0,
+        launchPDL(k_features<float, float>, dim3(nb0), dim3(kThreads), 0, s, nullptr, 0, N0_, smp.b, smp.AC, nullptr, nullptr, 0,
                                                           smp.deficit, scal_, (float*)feat_);
     forward(nullptr, 0, true, s);
     if (actBf16_)
-        k_loss_spmv<bfloat><<<nb0, kThreads, 0, s>>>(N0_, W0_, nb0_, smp.AF, smp.AC, (const bfloat*)out_, smp.b,
+        launchPDL(k_loss_spmv<bfloat>, dim3(nb0), dim3(kThreads), 0, s, N0_, W0_, nb0_, smp.AF, smp.AC, (const bfloat*)out_, smp.b,
                                                      smp.target, Ay_, red_, counter_, scal_);
     else
-        k_loss_spmv<float><<<nb0, kThreads, 0, s>>>(N0_, W0_, nb0_, smp.AF, smp.AC, (const float*)out_, smp.b,
+        launchPDL(k_loss_spmv<float>, dim3(nb0), dim3(kThreads), 0, s, N0_, W0_, nb0_, smp.AF, smp.AC, (const float*)out_, smp.b,
                                                     smp.target, Ay_, red_, counter_, scal_);
-    k_loss_grad<<<nb0, kThreads, 0, s>>>(N0_, smp.b, Ay_, scal_, gOut_, lossOut);
+    launchPDL(k_loss_grad, dim3(nb0), dim3(kThreads), 0, s, N0_, smp.b, Ay_, scal_, gOut_, lossOut);
     // zero every activation gradient except the output's, and the parameter gradient
     NCK(cudaMemsetAsync(gActs_, 0, gradActs_ * sizeof(float), s));
     NCK(cudaMemsetAsync(grad_, 0, nParams_ * sizeof(float), s));
@@ -1749,17 +1774,17 @@ void LearnedNet::lossAndGrad(const Sample& smp, float* lossOut, cudaStream_t s) 
 
 void LearnedNet::predict(const float* r, const float* AC, const float* deficit, float* out, cudaStream_t s) {
     const int nb0 = blocksFor(N0_);
-    k_sigma<float><<<nb0, kThreads, 0, s>>>(nullptr, 0, N0_, r, AC, red_, counter_, scal_);
+    launchPDL(k_sigma<float>, dim3(nb0), dim3(kThreads), 0, s, nullptr, 0, N0_, r, AC, red_, counter_, scal_);
     if (actBf16_) {
-        k_features<bfloat, float><<<nb0, kThreads, 0, s>>>(nullptr, 0, N0_, r, AC, nullptr, nullptr, 0, deficit, scal_,
+        launchPDL(k_features<bfloat, float>, dim3(nb0), dim3(kThreads), 0, s, nullptr, 0, N0_, r, AC, nullptr, nullptr, 0, deficit, scal_,
                                                            (bfloat*)feat_);
         forward(nullptr, 0, false, s);
-        k_scale_out<bfloat><<<nb0, kThreads, 0, s>>>(nullptr, 0, N0_, (const bfloat*)out_, scal_, out);
+        launchPDL(k_scale_out<bfloat>, dim3(nb0), dim3(kThreads), 0, s, nullptr, 0, N0_, (const bfloat*)out_, scal_, out);
     } else {
-        k_features<float, float><<<nb0, kThreads, 0, s>>>(nullptr, 0, N0_, r, AC, nullptr, nullptr, 0, deficit, scal_,
+        launchPDL(k_features<float, float>, dim3(nb0), dim3(kThreads), 0, s, nullptr, 0, N0_, r, AC, nullptr, nullptr, 0, deficit, scal_,
                                                           (float*)feat_);
         forward(nullptr, 0, false, s);
-        k_scale_out<float><<<nb0, kThreads, 0, s>>>(nullptr, 0, N0_, (const float*)out_, scal_, out);
+        launchPDL(k_scale_out<float>, dim3(nb0), dim3(kThreads), 0, s, nullptr, 0, N0_, (const float*)out_, scal_, out);
     }
     NCK(cudaGetLastError());
 }
@@ -1769,11 +1794,11 @@ void LearnedNet::trainStep(const Sample& smp, float lr, int t, float* lossOut, c
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)t), c2 = 1.f - std::pow(b2, (float)t);
     if (wBf16_)
-        k_adam<bfloat><<<blocksFor(nParams_), kThreads, 0, s>>>(nParams_, params_, grad_, adamM_, adamV_,
+        launchPDL(k_adam<bfloat>, dim3(blocksFor(nParams_)), dim3(kThreads), 0, s, nParams_, params_, grad_, adamM_, adamV_,
                                                                 (bfloat*)paramsLow_, lr, b1, b2, 1e-8f, c1, c2);
     if (wBf16_) packWeights(s);
     else
-        k_adam<float><<<blocksFor(nParams_), kThreads, 0, s>>>(nParams_, params_, grad_, adamM_, adamV_, params_, lr,
+        launchPDL(k_adam<float>, dim3(blocksFor(nParams_)), dim3(kThreads), 0, s, nParams_, params_, grad_, adamM_, adamV_, params_, lr,
                                                                b1, b2, 1e-8f, c1, c2);
     NCK(cudaGetLastError());
 }
