@@ -324,6 +324,7 @@ bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::
     for (int i = 0; i < plan.count; i++) {
         const GridLevel& g = hier[(size_t)(first + i)];
         const int N = g.nCells, R = plan.solo[i] ? N : 32 * ((N + 32 * chunks - 1) / (32 * chunks));
+        std::vector<int> seen((size_t)N, -1);  // the last CTA that has the cell in its halo
         for (int r = 0; r < plan.ctas; r++) {
             if (plan.solo[i] != (r == 0)) continue;
             Part& p = parts[(size_t)i][(size_t)r];
@@ -333,10 +334,11 @@ bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::
             p.s1 = p.n1 > p.n0 ? (p.n1 + 31) / 32 : p.s0;
             for (int k = g.faceStart[(size_t)p.n0]; k < g.faceStart[(size_t)p.n1]; k++) {
                 const int m = g.faceNeighbor[(size_t)k];
-                if (m >= 0 && (m < p.n0 || m >= p.n1)) p.halo.push_back(m);
+                if (m < 0 || (m >= p.n0 && m < p.n1) || seen[(size_t)m] == r) continue;
+                seen[(size_t)m] = r;
+                p.halo.push_back(m);
             }
             std::sort(p.halo.begin(), p.halo.end());
-            p.halo.erase(std::unique(p.halo.begin(), p.halo.end()), p.halo.end());
         }
     }
     // The solo levels and the chunks' levels share the same range of offsets:
@@ -395,6 +397,7 @@ bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::
     }
     if (plan.shared64 > kClusterMaxShared) return false;
     blob.assign((size_t)plan.blobBytes * (size_t)plan.ctas, 0);
+    std::vector<uint16_t> at(kClusterMaxCells);  // a halo cell's place on the CTA at hand
     for (int r = 0; r < plan.ctas; r++) {
         unsigned char* base = blob.data() + (size_t)r * plan.blobBytes;
         for (int i = 0; i < plan.count; i++) {
@@ -404,10 +407,8 @@ bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::
             std::memcpy(base + sizeof(ClusterRows) * (size_t)i, &l, sizeof l);
             if (l.rows == 0) continue;
             const std::vector<int32_t>& so = sliceOff[(size_t)(first + i)];
-            auto local = [&](int m) {
-                if (m >= p.n0 && m < p.n1) return m - p.n0;
-                return l.rows + (int)(std::lower_bound(p.halo.begin(), p.halo.end(), m) - p.halo.begin());
-            };
+            for (size_t k = 0; k < p.halo.size(); k++) at[(size_t)p.halo[k]] = (uint16_t)(l.rows + (int)k);
+            auto local = [&](int m) { return m >= p.n0 && m < p.n1 ? m - p.n0 : (int)at[(size_t)m]; };
             uint16_t* nb = reinterpret_cast<uint16_t*>(base + l.nb);
             for (int k = 0; k < l.slots; k++) nb[k] = (uint16_t)(l.cells - 1);
             for (int n = p.n0; n < p.n1; n++)
@@ -421,6 +422,7 @@ bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::
                         (uint32_t)(so[(size_t)k] - l.slot0) | (uint32_t)((so[(size_t)k + 1] - so[(size_t)k]) / 256) << 24;
             std::memcpy(base + l.halo, p.halo.data(), sizeof(int32_t) * p.halo.size());
             std::vector<int32_t> cells;  // rows, halo
+            cells.reserve((size_t)l.live);
             for (int n = p.n0; n < p.n1; n++) cells.push_back(n);
             cells.insert(cells.end(), p.halo.begin(), p.halo.end());
             if (i + 1 < plan.count)
