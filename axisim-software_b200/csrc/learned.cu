@@ -21,8 +21,9 @@
 // thousand rows. So the finest levels are bound by memory traffic and the
 // coarse ones by the latency of one tile; the products run as mma.sync on
 // operands that go from global memory straight into fragments
-// (k_layer_mma, k_layer_dz_mma; BF16 weights) or through shared-memory tiles
-// (k_layer_tile, k_layer_dz_tile; FP32 weights, the gradient check's mode).
+// (k_layer_mma, k_layer_dz_mma; predictions and input gradients with BF16
+// weights) or through shared-memory tiles (k_layer_tile, k_layer_dz_tile; the
+// solver's preconditioner, the training forward pass, and FP32 weights).
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -661,7 +662,6 @@ __global__ void __launch_bounds__(kMmaThreads) k_layer_mma(const Ctl* ctl, int g
     const bfloat* bias = P + L.wOff + (size_t)K * Cout;
     const TA* add = (const TA*)L.add;
     TA* Y = (TA*)L.Y;
-    TA* Z = col0 == 0 ? (TA*)L.Z : nullptr;
     const int tiles = (L.N + 15) / 16;
     for (int tile = blockIdx.x * perCta + warp / groups; tile < tiles; tile += gridDim.x * perCta) {
         const int r0 = tile * 16 + g, r1 = r0 + 8;
@@ -711,10 +711,6 @@ __global__ void __launch_bounds__(kMmaThreads) k_layer_mma(const Ctl* ctl, int g
                 } else {
                     va = ldv4(x + (size_t)ka[0] * C);
                     vb = ldv4(x + (size_t)kb[0] * C);
-                }
-                if (Z) {
-                    if (r0 < L.N) stv4(Z + (size_t)r0 * K + k0 + 4 * t4, va);
-                    if (r1 < L.N) stv4(Z + (size_t)r1 * K + k0 + 4 * t4, vb);
                 }
                 slabMma<NB>(acc, va, vb, w0 + (k0 / 16) * slabW);
             }
@@ -1657,10 +1653,20 @@ void LearnedNet::packWeights(cudaStream_t s) {
     if (a.n) launchPDL(k_pack, dim3(dim3(16, a.n)), dim3(kThreads), 0, s, a, (const bfloat*)paramsLow_, (bfloat*)packF_, (bfloat*)packB_);
 }
 
+// Predictions run on fragments from memory (874k cells: 0.8 ms of device time
+// against 1.76 with the tiles). The preconditioner inside a solve and the
+// training pass keep the tiles' rounding: a solve's FP64 iterates carry the
+// difference of two forward passes (1e-6) to 8e-6 of the fields, and the
+// gradient, a small difference of large sums, to 2.7e-5 (1.2e-5 to 1.6e-5 with
+// the tiles, from the weight gradient's shorter sums). Their price: a gradient
+// on 218k cells 1.6 -> 1.9 ms.
 void LearnedNet::forward(const Ctl* ctl, int gated, bool keepZ, cudaStream_t s) {
+    const bool tiles = ctl || keepZ;
     for (NetLayer L : layers_) {
         if (!keepZ) L.Z = nullptr;
-        if (actBf16_) launchLayerLow<bfloat>(ctl, gated, L, (const bfloat*)paramsLow_, (const bfloat*)packF_, s);
+        if (tiles && actBf16_) launchLayerFwd<bfloat, bfloat>(ctl, gated, L, paramsLow_, s);
+        else if (tiles && wBf16_) launchLayerFwd<float, bfloat>(ctl, gated, L, paramsLow_, s);
+        else if (actBf16_) launchLayerLow<bfloat>(ctl, gated, L, (const bfloat*)paramsLow_, (const bfloat*)packF_, s);
         else if (wBf16_) launchLayerLow<float>(ctl, gated, L, (const bfloat*)paramsLow_, (const bfloat*)packF_, s);
         else launchLayerFwd<float, float>(ctl, gated, L, paramsLow_, s);
     }
