@@ -722,8 +722,8 @@ class Solver:
         return dict(applied=a.value, fallbacks=f.value, score_net=sn.value, score_vcycle=sv.value)
 
     def set_momentum_sweeps(self, sweeps_per_launch, threads=0):
-        """Momentum Jacobi sweeps per launch (default 1 = one launch per sweep; above 1 run
-        on shared-memory tiles) and the CTA size of the tiled launches (0 = 1024)."""
+        """Momentum Jacobi sweeps per launch (default 1 = one launch per sweep, or all sweeps in
+        one launch on systems of up to 16,384 cells; above 1 run on shared-memory tiles) and the CTA size of the tiled launches (0 = 1024)."""
         self._check(lib().axisim_set_momentum_sweeps(self.h, sweeps_per_launch, threads))
 
     def sweep_tiles(self):

@@ -9,10 +9,12 @@
 //   * the fine residual is a coalesced pass over the fine level; the gather of
 //     the coarse right-hand side also performs the coarse level's first
 //     pre-smoothing sweep (from x = 0 it needs no neighbour values);
-//   * every level at or below 1024 cells runs as ONE single-CTA kernel holding
-//     x, the Jacobi partner, b and the residual in shared memory, with the
-//     coefficients L1-resident and the coarsest rows in registers (the
-//     reference launches three to four kernels per level per cycle there).
+//   * the levels of at most 15,360 cells run as one cluster launch
+//     (mg_cluster.cu); inside the resident V-cycle, and where the cluster's
+//     plan does not fit, those of at most 1024 cells run as one single-CTA
+//     kernel with x, the Jacobi partner, b and the residual in shared memory
+//     and the coarsest rows in registers (the reference launches three to
+//     four kernels per level per cycle there).
 // Every kernel is a template on the value type: double for the FP64 path
 // (compiled with --fmad=false, bit-exact with the CPU oracle), float for the
 // inner cycles of the mixed-precision path.

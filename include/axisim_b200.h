@@ -457,7 +457,7 @@ typedef struct axisim_kernel_stat {
 int axisim_profile_iteration(axisim_handle* h, int32_t iterations, axisim_kernel_stat* out, int32_t maxOut,
                              int32_t* nOut);
 /* As axisim_profile_iteration, with every multigrid launch (smoothing,
- * residual, restriction, prolongation, Galerkin, the one-CTA tail) named
+ * residual, restriction, prolongation, Galerkin, the deep levels' launch) named
  * "<kernel>@<level>" for a per-level breakdown of the V-cycle. */
 int axisim_profile_levels(axisim_handle* h, int32_t iterations, axisim_kernel_stat* out, int32_t maxOut,
                           int32_t* nOut);
