@@ -45,6 +45,7 @@ EXPORTS = [
     "axisim_set_autotune", "axisim_autotune_report", "axisim_setup_profile", "axisim_profile_levels",
     "axisim_mg_batch_levels_host", "axisim_set_vcycle_kernel", "axisim_test_barrier_timeout",
     "axisim_set_momentum_sweeps", "axisim_sweep_tiles", "axisim_sweep_tiles_host", "axisim_mesh_segments",
+    "axisim_vcycle_cluster_host",
 ]
 VAR_U, VAR_V, VAR_P, VAR_T, VAR_C = range(5)
 VAR_INDEX = {"u": VAR_U, "v": VAR_V, "p": VAR_P, "T": VAR_T, "C": VAR_C}
@@ -211,6 +212,8 @@ def lib():
             "axisim_mg_levels_host": (C.c_int, [C.POINTER(MeshPacked), _i32p, C.c_int32]),
             "axisim_mg_batch_levels_host": (C.c_int, [C.POINTER(MeshPacked), C.c_int32, _i32p, _i32p, _i32p,
                                                       C.c_int32]),
+            "axisim_vcycle_cluster_host": (C.c_int64, [C.POINTER(MeshPacked), C.c_int32, _i32p, C.c_int32, C.c_int32,
+                                                       C.c_int32, _i32p, _i32p, C.c_int32, _u8p, C.c_int64]),
             "axisim_mg_level_maps_host": (C.c_int64, [C.POINTER(MeshPacked), C.c_int32, vp, vp, vp, vp]),
             "axisim_coloring_host": (C.c_int, [C.POINTER(MeshPacked), _i32p, C.c_size_t]),
             "axisim_profile_iteration": (C.c_int, [vp, C.c_int32, C.POINTER(KernelStat), C.c_int32, _i32p]),
@@ -371,6 +374,31 @@ def mg_batch_levels_host(mesh, case_cell_start):
     if n < 0:
         raise AxisimError(-n, "mg_batch_levels_host failed")
     return cells[:n].copy(), term[:n].copy()
+
+
+def vcycle_cluster_host(mesh, case_cell_start=None, pre=1, post=1, coarse=30):
+    """The plan of the deep multigrid levels' cluster launch (axisim_vcycle_cluster_host):
+    None where a solve has none, else a dict of its first level, level count, ctas, threads,
+    steps (op, level, from, to, cluster-wide, flag) and the packed topology per CTA."""
+    s, keep = mesh_struct(mesh)
+    f = lib().axisim_vcycle_cluster_host
+    cs = None if case_cell_start is None else np.ascontiguousarray(case_cell_start, dtype=np.int32)
+    n = 0 if cs is None else len(cs) - 1
+    starts = None if cs is None else cs.ctypes.data_as(_i32p)
+    info = np.zeros(6, np.int32)
+    steps = np.zeros((256, 6), np.int32)
+    args = (C.byref(s), n, starts, pre, post, coarse, info.ctypes.data_as(_i32p), steps.ctypes.data_as(_i32p),
+            len(steps))
+    total = int(f(*args, None, 0))
+    if total < 0:
+        raise AxisimError(-total, "vcycle_cluster_host failed")
+    if total == 0:
+        return None
+    blob = np.zeros(total, np.uint8)
+    f(*args, blob.ctypes.data_as(_u8p), total)
+    first, count, ctas, threads, size, n_steps = (int(v) for v in info)
+    return dict(first=first, count=count, ctas=ctas, threads=threads, steps=steps[:n_steps].copy(),
+                blob=blob.reshape(ctas, size))
 
 
 def sweep_tiles_host(mesh, S, cap, tile_cells):

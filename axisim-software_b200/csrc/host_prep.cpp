@@ -816,6 +816,30 @@ std::vector<int32_t> slotNeighbours(int N, int W, const int32_t* cfs, const int3
     return nb;
 }
 
+std::vector<int32_t> sliceOffsets(const GridLevel& g, int group) {
+    const int n = (g.nCells + 31) / 32;
+    std::vector<int32_t> off((size_t)n + 1, 0);
+    for (int k = 0; k < n; k++) {
+        int w = 0;
+        for (int c = k * 32; c < std::min(g.nCells, k * 32 + 32); c++)
+            w = std::max(w, g.faceStart[(size_t)c + 1] - g.faceStart[(size_t)c]);
+        off[(size_t)k + 1] = off[(size_t)k] + 32 * ((w + group - 1) / group * group);
+    }
+    return off;
+}
+
+void coarseMembers(const GridLevel& fine, const GridLevel& coarse, std::vector<int32_t>& start,
+                   std::vector<int32_t>& list) {
+    start.assign((size_t)coarse.nCells + 1, 0);
+    for (int n = 0; n < fine.nCells; n++)
+        if (fine.cellToCoarse[(size_t)n] >= 0) start[(size_t)fine.cellToCoarse[(size_t)n] + 1]++;
+    for (int k = 0; k < coarse.nCells; k++) start[(size_t)k + 1] += start[(size_t)k];
+    list.assign((size_t)std::max(start[(size_t)coarse.nCells], 1), 0);
+    std::vector<int32_t> fill(start);
+    for (int n = 0; n < fine.nCells; n++)
+        if (fine.cellToCoarse[(size_t)n] >= 0) list[(size_t)fill[(size_t)fine.cellToCoarse[(size_t)n]]++] = n;
+}
+
 // The cells along a Morton curve of their centres: exact within buckets of more
 // than `refine` cells, by cell id within smaller ones.
 static std::vector<int32_t> curveOrder(int N, const double* cz, const double* cr, int refine) {

@@ -120,6 +120,14 @@ std::vector<GridLevel> buildHierarchy(GridLevel finest);
 std::vector<GridLevel> buildBatchHierarchy(const GridLevel& finest, const std::vector<int32_t>& caseStart,
                                            std::vector<std::vector<int32_t>>& terminal);
 
+// Offsets of a coarse level's 32-row slices in sliced ELL: each as wide as its
+// longest row, rounded up to a multiple of `group` slots.
+std::vector<int32_t> sliceOffsets(const GridLevel& g, int group);
+// Members of each coarse cell in ascending order, as start + list (a batch's
+// terminal cells have no coarse cell).
+void coarseMembers(const GridLevel& fine, const GridLevel& coarse, std::vector<int32_t>& start,
+                   std::vector<int32_t>& list);
+
 // Tiles for running several momentum Jacobi sweeps (linear_solver.cu:9-33)
 // per launch out of shared memory. Cells are ordered along a Morton curve of
 // their centres (one scale for both axes) and cut into runs of `tileCells`

@@ -104,6 +104,7 @@ constexpr int kClusterSize = 16;
 constexpr int kMaxClusterLevels = 10;
 constexpr int kClusterMaxCells = 15 * 1024;
 constexpr int kClusterSolo = 1024;
+constexpr int kClusterThreads = 512;  // kClCoarsest takes levels of at most this many rows, one a thread
 constexpr size_t kClusterMaxShared = 220 * 1024;
 // A level on one CTA: its rows from global cell row0, and offsets into the
 // CTA's shared memory. Cells are numbered rows, halo, padding, zero cell.
@@ -119,7 +120,7 @@ struct MgClusterPlan {
     uint32_t blobBytes = 0;               // per CTA
     const unsigned char* blob = nullptr;  // device, one block per CTA: its ClusterRows, then what they point to
     size_t shared64 = 0, shared32 = 0;
-    int32_t W[kMaxClusterLevels] = {};
+    int32_t W[kMaxClusterLevels] = {}, N[kMaxClusterLevels] = {};
     bool solo[kMaxClusterLevels] = {};
 };
 enum ClusterOp : uint8_t { kClSweep, kClResidual, kClRestrict, kClCorrect, kClHalo, kClCoarsest, kClStore };
@@ -132,12 +133,19 @@ struct ClusterStep {
 };
 constexpr int kMaxClusterSteps = 64;
 struct GridLevel;
-// The plan of levels first.. and the packed topology of its CTAs; false when
-// they do not fit (a level above kClusterMaxCells, too many levels, shared
-// memory). sliceOff, mStart, mList: the levels' slice offsets and member lists.
-bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::vector<std::vector<int32_t>>& sliceOff,
-                      const std::vector<std::vector<int32_t>>& mStart, const std::vector<std::vector<int32_t>>& mList,
-                      MgClusterPlan& plan, std::vector<unsigned char>& blob);
+// Slots a row of a coarse level is padded to a multiple of: eight where the
+// level can be in a cluster.
+inline int sliceGroup(int cells) { return cells <= kClusterMaxCells ? 8 : 1; }
+// The plan from the finest level below the last terminal one that allows it
+// (every level at most kClusterMaxCells, at most kMaxClusterLevels of them,
+// shared memory) and the packed topology of its CTAs; first < 0: none.
+// sliceOff, mStart, mList: the levels' slice offsets and member lists.
+MgClusterPlan findClusterPlan(const std::vector<GridLevel>& hier, int lastTerminal,
+                              const std::vector<std::vector<int32_t>>& sliceOff,
+                              const std::vector<std::vector<int32_t>>& mStart,
+                              const std::vector<std::vector<int32_t>>& mList, std::vector<unsigned char>& blob);
+// The steps of a cycle on the plan's levels, without their addresses (none: too many).
+std::vector<ClusterStep> clusterStepList(const MgClusterPlan& plan, int pre, int post, int coarse);
 bool clusterRunnable(const MgClusterPlan& plan);
 template <class T>
 struct ClusterArgsT {

@@ -43,8 +43,6 @@ namespace axisim {
 
 namespace {
 
-constexpr int kClusterThreads = 512;
-
 inline size_t align16(size_t n) { return (n + 15) & ~size_t(15); }
 
 template <class T>
@@ -296,7 +294,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_mg_cluster(const Ctl* ct
 }  // namespace
 
 // ---- host: the plan of a hierarchy and its packed topology ----
-bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::vector<std::vector<int32_t>>& sliceOff,
+static bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::vector<std::vector<int32_t>>& sliceOff,
                       const std::vector<std::vector<int32_t>>& mStart, const std::vector<std::vector<int32_t>>& mList,
                       MgClusterPlan& plan, std::vector<unsigned char>& blob) {
     plan = MgClusterPlan();
@@ -312,6 +310,7 @@ bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::
         const std::vector<int32_t>& so = sliceOff[(size_t)(first + i)];
         for (size_t k = 0; k + 1 < so.size(); k++) W = std::max(W, (so[k + 1] - so[k]) / 32);
         plan.W[i] = W;
+        plan.N[i] = N;
     }
     plan.ctas = plan.solo[0] ? 1 : kClusterSize;  // CTA 0: the solo levels; the others: the chunks
     const int chunks = kClusterSize - 1;
@@ -445,6 +444,16 @@ bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, const std::
     return true;
 }
 
+MgClusterPlan findClusterPlan(const std::vector<GridLevel>& hier, int lastTerminal,
+                              const std::vector<std::vector<int32_t>>& sliceOff,
+                              const std::vector<std::vector<int32_t>>& mStart,
+                              const std::vector<std::vector<int32_t>>& mList, std::vector<unsigned char>& blob) {
+    MgClusterPlan plan;
+    for (int t = std::max(1, lastTerminal + 1); t < (int)hier.size(); t++)
+        if (buildClusterPlan(hier, t, sliceOff, mStart, mList, plan, blob)) return plan;
+    return MgClusterPlan();
+}
+
 template <class T>
 static cudaLaunchConfig_t clusterConfig(const MgClusterPlan& plan, cudaLaunchAttribute (&attr)[2]) {
     cudaLaunchConfig_t cfg = {};
@@ -528,7 +537,9 @@ static bool clusterSteps(ClusterArgsT<T>& a) {
         add(kClRestrict, i + 1, cur[i] ^ 1, 0, r, nullptr, firstDone ? 1 : 0, false);
     }
     const int sweeps = a.coarse - (firstDone ? 1 : 0);
-    if (p.solo[last] && p.W[last] <= 8 && sweeps > 0) {
+    // A batch merges its cases' coarsest levels, so this one can have more rows
+    // than the CTA has threads: it is swept like any other level then.
+    if (p.solo[last] && p.N[last] <= kClusterThreads && p.W[last] <= 8 && sweeps > 0) {
         add(kClCoarsest, last, cur[last], 0, nullptr, nullptr, sweeps, false);
         cur[last] ^= sweeps & 1;
     } else {
@@ -545,6 +556,18 @@ static bool clusterSteps(ClusterArgsT<T>& a) {
     }
     if (p.solo[0]) add(kClStore, 0, cur[0], 0, a.x[0][0], nullptr, 0, false);
     return a.nSteps <= kMaxClusterSteps;
+}
+
+std::vector<ClusterStep> clusterStepList(const MgClusterPlan& plan, int pre, int post, int coarse) {
+    ClusterArgsT<double> a;
+    a.plan = plan;
+    a.pre = pre;
+    a.post = post;
+    a.coarse = coarse;
+    double anywhere = 0.0;  // a step reads or writes L2 where it has an address
+    for (int i = 0; i < kMaxClusterLevels; i++) a.x[i][0] = a.x[i][1] = a.res[i] = &anywhere;
+    if (!clusterSteps(a)) return {};
+    return std::vector<ClusterStep>(a.steps, a.steps + a.nSteps);
 }
 
 template <class T>

@@ -1222,20 +1222,12 @@ private:
                 d.x = pp_;
                 d.xNew = ppT_;
             } else {
-                const int nS = (g.nCells + 31) / 32;
                 std::vector<int32_t>& off = sliceOffH[(size_t)l];
-                off.assign((size_t)nS + 1, 0);
+                off = sliceOffsets(g, sliceGroup(g.nCells));
                 int W = 0;
-                for (int sI = 0; sI < nS; sI++) {
-                    int w = 0;
-                    for (int c = sI * 32; c < std::min(g.nCells, sI * 32 + 32); c++)
-                        w = std::max(w, g.faceStart[(size_t)c + 1] - g.faceStart[(size_t)c]);
-                    if (g.nCells <= kClusterMaxCells) w = (w + 7) & ~7;  // groups of eight slots (mg_cluster.cu)
-                    off[(size_t)sI + 1] = off[(size_t)sI] + 32 * w;
-                    W = std::max(W, w);
-                }
+                for (size_t k = 0; k + 1 < off.size(); k++) W = std::max(W, (off[k + 1] - off[k]) / 32);
                 d.W = W;
-                d.totalSlots = off[(size_t)nS];
+                d.totalSlots = off.back();
                 std::vector<int32_t> nb((size_t)std::max(d.totalSlots, 1), -1);
                 parallelFor(g.nCells, [&](int c0, int c1) {
                     for (int c = c0; c < c1; c++)
@@ -1261,17 +1253,8 @@ private:
             const GridLevel& c = hier_[(size_t)l];
             LevelDev& fd = levels_[(size_t)l - 1];
             LevelDev& cd = levels_[(size_t)l];
-            // members of each coarse cell (a batch's terminal cells have no coarse cell)
-            std::vector<int32_t> mStart((size_t)c.nCells + 1, 0), mList;
-            for (int n = 0; n < f.nCells; n++)
-                if (f.cellToCoarse[(size_t)n] >= 0) mStart[(size_t)f.cellToCoarse[(size_t)n] + 1]++;
-            for (int k = 0; k < c.nCells; k++) mStart[(size_t)k + 1] += mStart[(size_t)k];
-            mList.resize((size_t)std::max(mStart[(size_t)c.nCells], 1));
-            {
-                std::vector<int32_t> fill(mStart);
-                for (int n = 0; n < f.nCells; n++)
-                    if (f.cellToCoarse[(size_t)n] >= 0) mList[(size_t)fill[(size_t)f.cellToCoarse[(size_t)n]]++] = n;
-            }
+            std::vector<int32_t> mStart, mList;
+            coarseMembers(f, c, mStart, mList);
             std::vector<int32_t> coarsePos((size_t)std::max(c.nFaceRefs(), 1));
             parallelFor(c.nCells, [&](int c0, int c1) {
                 for (int cc = c0; cc < c1; cc++)
@@ -1347,16 +1330,10 @@ private:
             }
         }
         // the finest level from which on all fit one thread-block cluster
-        cluster_ = MgClusterPlan();
-        for (int t = std::max(1, lastTerminal + 1); t < L; t++) {
-            MgClusterPlan plan;
-            std::vector<unsigned char> blob;
-            if (!buildClusterPlan(hier_, t, sliceOffH, mStartH, mListH, plan, blob)) continue;
-            if (!clusterRunnable(plan)) break;
-            plan.blob = mgArena_.upload(blob.data(), blob.size());
-            cluster_ = plan;
-            break;
-        }
+        std::vector<unsigned char> blob;
+        cluster_ = findClusterPlan(hier_, lastTerminal, sliceOffH, mStartH, mListH, blob);
+        if (cluster_.first >= 0 && !clusterRunnable(cluster_)) cluster_ = MgClusterPlan();
+        if (cluster_.first >= 0) cluster_.blob = mgArena_.upload(blob.data(), blob.size());
     }
     int tailStart_ = -1;
     MgClusterPlan cluster_;  // first < 0: none
@@ -3472,6 +3449,49 @@ int axisim_mg_batch_levels_host(const axisim_mesh_packed* mesh, int32_t nCases, 
             terminalCellsPerLevel[l] = t;
         }
         return (int)h.size();
+    } catch (...) {
+        return -AXISIM_E_MESH;
+    }
+}
+
+int64_t axisim_vcycle_cluster_host(const axisim_mesh_packed* mesh, int32_t nCases, const int32_t* caseCellStart,
+                                   int32_t preSweeps, int32_t postSweeps, int32_t coarseSweeps, int32_t* info,
+                                   int32_t* steps, int32_t maxSteps, unsigned char* blob, int64_t blobCapacity) {
+    if (!info || maxSteps < 0 || (maxSteps > 0 && !steps) || nCases < 0 || (nCases > 0 && !caseCellStart))
+        return -AXISIM_E_ARG;
+    if (!connectivityOk(mesh)) return -AXISIM_E_MESH;
+    if (nCases > 0 && (caseCellStart[0] != 0 || caseCellStart[nCases] != mesh->nCells)) return -AXISIM_E_ARG;
+    for (int c = 0; c < nCases; c++)
+        if (caseCellStart[c + 1] <= caseCellStart[c]) return -AXISIM_E_ARG;
+    try {
+        using namespace axisim;
+        std::vector<std::vector<int32_t>> term;
+        std::vector<GridLevel> h;
+        if (nCases > 0)
+            h = buildBatchHierarchy(hostFinest(mesh), std::vector<int32_t>(caseCellStart, caseCellStart + nCases + 1), term);
+        else
+            h = buildHierarchy(hostFinest(mesh));
+        int lastTerminal = -1;
+        for (size_t l = 0; l < term.size(); l++)
+            if (!term[l].empty()) lastTerminal = (int)l;
+        std::vector<std::vector<int32_t>> so(h.size()), ms(h.size()), ml(h.size());
+        for (size_t l = 1; l < h.size(); l++) {
+            so[l] = sliceOffsets(h[l], sliceGroup(h[l].nCells));
+            coarseMembers(h[l - 1], h[l], ms[l], ml[l]);
+        }
+        std::vector<unsigned char> b;
+        const MgClusterPlan p = findClusterPlan(h, lastTerminal, so, ms, ml, b);
+        std::fill(info, info + 6, 0);
+        if (p.first < 0) return 0;
+        const std::vector<ClusterStep> list = clusterStepList(p, preSweeps, postSweeps, coarseSweeps);
+        const int32_t v[6] = {p.first, p.count, p.ctas, kClusterThreads, (int32_t)p.blobBytes, (int32_t)list.size()};
+        std::copy(v, v + 6, info);
+        for (size_t k = 0; k < list.size() && (int)k < maxSteps; k++) {
+            const int32_t f[6] = {list[k].op, list[k].level, list[k].from, list[k].to, list[k].clusterWide, list[k].flag};
+            std::copy(f, f + 6, steps + 6 * k);
+        }
+        if (blob && blobCapacity >= (int64_t)b.size()) std::copy(b.begin(), b.end(), blob);
+        return (int64_t)b.size();
     } catch (...) {
         return -AXISIM_E_MESH;
     }

@@ -422,6 +422,17 @@ int axisim_mg_levels_host(const axisim_mesh_packed* mesh, int32_t* cellsPerLevel
  * (0 on the deepest level). Returns the number of levels or -status. */
 int axisim_mg_batch_levels_host(const axisim_mesh_packed* mesh, int32_t nCases, const int32_t* caseCellStart,
                                 int32_t* cellsPerLevel, int32_t* terminalCellsPerLevel, int32_t maxLevels);
+/* New: the plan by which a solve of this mesh (nCases > 0: of a batch with these
+ * case ranges) runs its deep multigrid levels as one thread-block cluster, for
+ * inspection without a device. info[6]: first level, levels, CTAs, threads a
+ * CTA, bytes a CTA of the packed topology, steps of a cycle with these sweep
+ * counts (all 0: no plan; no steps: more than fit, the cycle runs without the
+ * plan). steps: op, level, from, to, cluster-wide, flag of
+ * each. Returns the bytes of the topology, copied to blob where they fit, or
+ * -status. */
+int64_t axisim_vcycle_cluster_host(const axisim_mesh_packed* mesh, int32_t nCases, const int32_t* caseCellStart,
+                                   int32_t preSweeps, int32_t postSweeps, int32_t coarseSweeps, int32_t* info,
+                                   int32_t* steps, int32_t maxSteps, unsigned char* blob, int64_t blobCapacity);
 int64_t axisim_mg_level_maps_host(const axisim_mesh_packed* mesh, int32_t level, int32_t* cellToCoarse,
                                   int32_t* fineSlotToCoarseSlot, int32_t* coarseFaceStart,
                                   int32_t* coarseFaceNeighbor);

@@ -1,0 +1,42 @@
+"""Batches whose cases' coarsest levels, merged, are larger than the deep levels'
+cluster has threads (needs a B200): every case equals its standalone solve bit
+for bit, in FP64 and mixed precision, on both sides of 512 and of 1,024 rows.
+"""
+import numpy as np
+import pytest
+
+from axisim import batch, cases
+import axisim.abi as abi
+from test_cluster_plan_cpu import BATCHES
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("u", "v", "p", "mDot")
+
+
+def _member(i, nr, nz):
+    c = cases.pipe(nr=nr, nz=nz, max_iter=2, tol=1e-30, U0=0.02 + 0.001 * i)
+    c.settings.update(linearType=cases.LINEAR_JACOBI)
+    return c
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("rows", list(BATCHES))
+def test_every_case_equals_its_own_solve(rows, precision):
+    sizes = [(nr, nz) for n, nr, nz in BATCHES[rows] for _ in range(n)]
+    members = [_member(i, *s) for i, s in enumerate(sizes)]
+    meshes = [abi.multiblock(c.blocks) for c in members]
+    union, start, bcs = batch.pack_union(meshes, [c.groups for c in members])
+    s = abi.Solver(union, bcs, members[0].settings, precision=precision)
+    s.set_batch(start)
+    s.solve()
+    got = {f: s.get(f) for f in FIELDS}
+    s.close()
+    faces = np.cumsum([0] + [m["nFaces"] for m in meshes])
+    for i in sorted({0, 1, len(members) // 2, len(members) - 1}):
+        one = abi.Solver(meshes[i], members[i].bc_fields(), members[i].settings, precision=precision)
+        one.solve()
+        for f in FIELDS:
+            at = faces if f == "mDot" else start
+            np.testing.assert_array_equal(got[f][at[i]:at[i + 1]], one.get(f), err_msg=f"{f} of case {i}")
+        one.close()
