@@ -823,7 +823,8 @@ std::vector<int32_t> sliceOffsets(const GridLevel& g, int group) {
         int w = 0;
         for (int c = k * 32; c < std::min(g.nCells, k * 32 + 32); c++)
             w = std::max(w, g.faceStart[(size_t)c + 1] - g.faceStart[(size_t)c]);
-        off[(size_t)k + 1] = off[(size_t)k] + 32 * ((w + group - 1) / group * group);
+        w = (w + group - 1) / group * group;
+        off[(size_t)k + 1] = off[(size_t)k] + 32 * (group > 1 ? std::max(w, group) : w);
     }
     return off;
 }

@@ -121,7 +121,8 @@ std::vector<GridLevel> buildBatchHierarchy(const GridLevel& finest, const std::v
                                            std::vector<std::vector<int32_t>>& terminal);
 
 // Offsets of a coarse level's 32-row slices in sliced ELL: each as wide as its
-// longest row, rounded up to a multiple of `group` slots.
+// longest row, rounded up to a multiple of `group` slots (at least one group
+// where there are groups, also for 32 rows without a neighbour).
 std::vector<int32_t> sliceOffsets(const GridLevel& g, int group);
 // Members of each coarse cell in ascending order, as start + list (a batch's
 // terminal cells have no coarse cell).

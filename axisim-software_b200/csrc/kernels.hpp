@@ -133,8 +133,8 @@ struct ClusterStep {
 };
 constexpr int kMaxClusterSteps = 64;
 struct GridLevel;
-// Slots a row of a coarse level is padded to a multiple of: eight where the
-// level can be in a cluster.
+// Slots a row of a coarse level is padded to a multiple of: eight (and at least
+// eight) where the level can be in a cluster.
 inline int sliceGroup(int cells) { return cells <= kClusterMaxCells ? 8 : 1; }
 // The plan from the finest level below the last terminal one that allows it
 // (every level at most kClusterMaxCells, at most kMaxClusterLevels of them,

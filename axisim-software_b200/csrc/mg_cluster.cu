@@ -20,8 +20,8 @@
 //     with the list of steps before the kernel waits for its predecessor; read
 //     from the kernel's parameters, each step's look-ups were a chain of
 //     constant-bank misses of about 1,000 cycles.
-//   * A row has its slots in groups of eight (the levels' slices are padded),
-//     so its loads have constant offsets. An unused slot refers to the chunk's
+//   * A row has its slots in groups of eight and at least one group (the levels'
+//     slices are padded), so its loads have constant offsets. An unused slot refers to the chunk's
 //     zero cell, which holds -0.0, and has the coefficient +0: its product is
 //     -0.0 and adding it leaves every sum as it is, bit for bit.
 //
@@ -308,7 +308,11 @@ static bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, cons
         if (i > 0 && plan.solo[i - 1] && !plan.solo[i]) return false;
         int W = 0;
         const std::vector<int32_t>& so = sliceOff[(size_t)(first + i)];
-        for (size_t k = 0; k + 1 < so.size(); k++) W = std::max(W, (so[k + 1] - so[k]) / 32);
+        for (size_t k = 0; k + 1 < so.size(); k++) {
+            const int w = (so[k + 1] - so[k]) / 32;
+            if (w < 8 || w % 8 != 0) return false;  // the kernel takes whole groups of eight, and one of every row
+            W = std::max(W, w);
+        }
         plan.W[i] = W;
         plan.N[i] = N;
     }

@@ -1,13 +1,16 @@
-"""Batches whose cases' coarsest levels, merged, are larger than the deep levels'
-cluster has threads (needs a B200): every case equals its standalone solve bit
-for bit, in FP64 and mixed precision, on both sides of 512 and of 1,024 rows.
+"""Cases in one mesh on the deep multigrid levels' cluster (needs a B200). Batches
+whose cases' coarsest levels, merged, are larger than it has threads: every case
+equals its standalone solve bit for bit, in FP64 and mixed precision, on both
+sides of 512 and of 1,024 rows. Small cases that share one hierarchy, with whole
+slices of isolated coarse cells: the oracle's fields bit for bit.
 """
 import numpy as np
 import pytest
 
 from axisim import batch, cases
 import axisim.abi as abi
-from test_cluster_plan_cpu import BATCHES
+import oracle
+from test_cluster_plan_cpu import BATCHES, SMALL, SORTED
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +43,19 @@ def test_every_case_equals_its_own_solve(rows, precision):
             at = faces if f == "mDot" else start
             np.testing.assert_array_equal(got[f][at[i]:at[i + 1]], one.get(f), err_msg=f"{f} of case {i}")
         one.close()
+
+
+@pytest.mark.parametrize("name", ["small", "sorted", "mixed"])
+def test_isolated_cells_match_the_oracle(name):
+    # cases that share one hierarchy: a case down to one cell is a coarse cell without a neighbour
+    sizes = {"small": SMALL, "sorted": SORTED, "mixed": [(2, 4)] * 40 + [(40, 200)]}[name]
+    members = [_member(i % 8, *s) for i, s in enumerate(sizes)]
+    union, _, bcs = batch.pack_union([abi.multiblock(c.blocks) for c in members], [c.groups for c in members])
+    gpu = abi.Solver(union, bcs, members[0].settings)
+    gpu.solve()
+    orc = oracle.Oracle(union, bcs, members[0].settings)
+    orc.run()
+    for f in FIELDS + ("pp",):
+        np.testing.assert_array_equal(gpu.get(f), orc.get(f), err_msg=f)
+    gpu.close()
+    orc.close()
