@@ -568,6 +568,7 @@ std::vector<ClusterStep> clusterStepList(const MgClusterPlan& plan, int pre, int
     a.pre = pre;
     a.post = post;
     a.coarse = coarse;
+    a.firstDone = (plan.count == 1 ? coarse : pre) >= 1 ? 1 : 0;  // the restriction into level `first` ran it
     double anywhere = 0.0;  // a step reads or writes L2 where it has an address
     for (int i = 0; i < kMaxClusterLevels; i++) a.x[i][0] = a.x[i][1] = a.res[i] = &anywhere;
     if (!clusterSteps(a)) return {};

@@ -1617,7 +1617,8 @@ private:
         const T w = (T)cmg_.weight;
         const char* tag = sizeof(T) == 8 ? "" : "32";
         const double vb = (double)sizeof(T);
-        if (l == cluster_.first && !residentVcycle_ && clusterCycle<T>(lv, cur, alt, firstDone)) return;
+        const int clusterAt = clusterLevel();
+        if (l == clusterAt && clusterCycle<T>(lv, cur, alt, firstDone)) return;
         if (hier_[(size_t)l].isCoarsest()) {
             smoothT<T>(lv, l, cmg_.linearSweep - (firstDone ? 1 : 0), cur, alt);
             return;
@@ -1629,7 +1630,7 @@ private:
         // itself (one launch instead of two where launches dominate); larger
         // levels, the finest one (coalesced [W][N] rows) and the level above
         // the tail (whose residual the tail reads) keep the separate pass
-        const bool tail = l + 1 == tailStart_ && (l + 1 != cluster_.first || residentVcycle_);
+        const bool tail = l + 1 == tailStart_ && l + 1 != clusterAt;
         const bool gatherRes = F.sliceOff != nullptr && F.N <= kFuseGatherCells && !tail;
         if (!gatherRes) {
             T* x = cur[(size_t)l];
@@ -1639,7 +1640,7 @@ private:
         }
         // level l + 1's operator is read from here on; the tail reads every
         // level below it as well
-        joinGalerkin(tail || l + 1 == cluster_.first ? L - 1 : l + 1);
+        joinGalerkin(tail || l + 1 == clusterAt ? L - 1 : l + 1);
         if (tail) {
             TailArgsT<T> a;
             a.first = l + 1;
@@ -1767,7 +1768,7 @@ private:
     template <class T>
     bool forkTerminal(std::vector<LevelT<T>>& lv, int l, T* x, T w) {
         const LevelT<T>& F = lv[(size_t)l];
-        const bool tailNext = l + 1 == tailStart_ && (l + 1 != cluster_.first || residentVcycle_);
+        const bool tailNext = l + 1 == tailStart_ && l + 1 != clusterLevel();
         if (profiling_ || psolve_ == AXISIM_PSOLVE_FCG || residentVcycle_ || cmg_.linearPreSweep > 1 ||
             hier_[(size_t)l].isCoarsest() || !F.sliceOff || F.N > kFuseGatherCells || tailNext)
             return false;
@@ -1789,6 +1790,15 @@ private:
         CK(cudaStreamWaitEvent(stream_, termFork_[(size_t)l].done, 0));
         termFork_[(size_t)l].open = false;
         tNextLaunchPlain = true;  // the next kernel follows the join
+    }
+
+    // The level from which on the cycle is one cluster launch, -1: none. Not in
+    // the resident V-cycle, and not with more sweeps than its list of steps
+    // holds: those cycles keep the per-phase launches and the tail.
+    int clusterLevel() const {
+        const bool fits = cluster_.first >= 0 && !residentVcycle_ &&
+                          !clusterStepList(cluster_, cmg_.linearPreSweep, cmg_.linearPostSweep, cmg_.linearSweep).empty();
+        return fits ? cluster_.first : -1;
     }
 
     // The cycle from the cluster's finest level down as one launch (in place in cur).
