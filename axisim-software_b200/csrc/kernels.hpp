@@ -104,7 +104,8 @@ constexpr int kClusterSize = 16;
 constexpr int kMaxClusterLevels = 10;
 constexpr int kClusterMaxCells = 15 * 1024;
 constexpr int kClusterSolo = 1024;
-constexpr int kClusterThreads = 512;  // kClCoarsest takes levels of at most this many rows, one a thread
+constexpr int kClusterThreads = 512;       // kClCoarsest takes levels of at most as many rows as the CTA has
+constexpr int kClusterThreadsLarge = 1024;  // threads, one a thread: more of them where a coarsest level is larger
 constexpr size_t kClusterMaxShared = 220 * 1024;
 // A level on one CTA: its rows from global cell row0, and offsets into the
 // CTA's shared memory. Cells are numbered rows, halo, padding, zero cell.
@@ -116,7 +117,7 @@ struct ClusterRows {
     uint32_t value64 = 0, value32 = 0;  // the level's values, by precision
 };
 struct MgClusterPlan {
-    int first = -1, count = 0, ctas = 0;
+    int first = -1, count = 0, ctas = 0, threads = kClusterThreads;
     uint32_t blobBytes = 0;               // per CTA
     const unsigned char* blob = nullptr;  // device, one block per CTA: its ClusterRows, then what they point to
     size_t shared64 = 0, shared32 = 0;

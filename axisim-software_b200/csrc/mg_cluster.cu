@@ -210,9 +210,9 @@ __device__ __forceinline__ void coarsestRows(const View<T>& L, uint32_t x, uint3
                       [&] { partSync(part); });
 }
 
-template <class T>
-__global__ void __launch_bounds__(kClusterThreads, 1) k_mg_cluster(const Ctl* ctl,
-                                                                   const __grid_constant__ ClusterArgsT<T> a) {
+template <class T, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_mg_cluster(const Ctl* ctl,
+                                                           const __grid_constant__ ClusterArgsT<T> a) {
     const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     const int rank = (int)cl.block_rank();
     // the packed block and the steps do not depend on earlier kernels
@@ -316,6 +316,9 @@ static bool buildClusterPlan(const std::vector<GridLevel>& hier, int first, cons
         plan.W[i] = W;
         plan.N[i] = N;
     }
+    const int last = plan.count - 1;
+    // one row a thread on a coarsest level of up to 1,024 rows (a batch's merged one)
+    if (plan.solo[last] && plan.W[last] <= 8 && plan.N[last] > kClusterThreads) plan.threads = kClusterThreadsLarge;
     plan.ctas = plan.solo[0] ? 1 : kClusterSize;  // CTA 0: the solo levels; the others: the chunks
     const int chunks = kClusterSize - 1;
     // a level on a CTA: its rows, its halo in ascending order, its slices
@@ -462,7 +465,7 @@ template <class T>
 static cudaLaunchConfig_t clusterConfig(const MgClusterPlan& plan, cudaLaunchAttribute (&attr)[2]) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(plan.ctas);
-    cfg.blockDim = dim3(kClusterThreads);
+    cfg.blockDim = dim3(plan.threads);
     cfg.dynamicSmemBytes = sizeof(T) == 8 ? plan.shared64 : plan.shared32;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = plan.ctas;
@@ -478,15 +481,20 @@ static cudaLaunchConfig_t clusterConfig(const MgClusterPlan& plan, cudaLaunchAtt
 // Whether the current device can hold the cluster of either precision (a GPC
 // with kClusterSize SMs free); also raises the kernels' limits on it.
 template <class T>
+static auto* clusterKernel(const MgClusterPlan& plan) {
+    return plan.threads == kClusterThreads ? k_mg_cluster<T, kClusterThreads> : k_mg_cluster<T, kClusterThreadsLarge>;
+}
+template <class T>
 static bool clusterFits(const MgClusterPlan& plan) {
+    auto* f = clusterKernel<T>(plan);
     cudaLaunchAttribute attr[2];
     const cudaLaunchConfig_t cfg = clusterConfig<T>(plan, attr);
     int n = 0;
     const bool ok =
-        cudaFuncSetAttribute(k_mg_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaFuncSetAttribute(k_mg_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterMaxShared) ==
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterMaxShared) ==
             cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&n, k_mg_cluster<T>, &cfg) == cudaSuccess && n >= 1;
+        cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n >= 1;
     cudaGetLastError();
     return ok;
 }
@@ -541,9 +549,7 @@ static bool clusterSteps(ClusterArgsT<T>& a) {
         add(kClRestrict, i + 1, cur[i] ^ 1, 0, r, nullptr, firstDone ? 1 : 0, false);
     }
     const int sweeps = a.coarse - (firstDone ? 1 : 0);
-    // A batch merges its cases' coarsest levels, so this one can have more rows
-    // than the CTA has threads: it is swept like any other level then.
-    if (p.solo[last] && p.N[last] <= kClusterThreads && p.W[last] <= 8 && sweeps > 0) {
+    if (p.solo[last] && p.N[last] <= p.threads && p.W[last] <= 8 && sweeps > 0) {
         add(kClCoarsest, last, cur[last], 0, nullptr, nullptr, sweeps, false);
         cur[last] ^= sweeps & 1;
     } else {
@@ -583,7 +589,7 @@ bool launchMGCluster(const Ctl* ctl, ClusterArgsT<T> a, cudaStream_t s) {
     cfg.stream = s;
     cfg.numAttrs = tNextLaunchPlain ? 1 : 2;
     tNextLaunchPlain = false;
-    return cudaLaunchKernelEx(&cfg, k_mg_cluster<T>, ctl, a) == cudaSuccess;
+    return cudaLaunchKernelEx(&cfg, clusterKernel<T>(a.plan), ctl, a) == cudaSuccess;
 }
 
 template bool launchMGCluster<double>(const Ctl*, ClusterArgsT<double>, cudaStream_t);

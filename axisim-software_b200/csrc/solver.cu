@@ -3494,7 +3494,7 @@ int64_t axisim_vcycle_cluster_host(const axisim_mesh_packed* mesh, int32_t nCase
         std::fill(info, info + 6, 0);
         if (p.first < 0) return 0;
         const std::vector<ClusterStep> list = clusterStepList(p, preSweeps, postSweeps, coarseSweeps);
-        const int32_t v[6] = {p.first, p.count, p.ctas, kClusterThreads, (int32_t)p.blobBytes, (int32_t)list.size()};
+        const int32_t v[6] = {p.first, p.count, p.ctas, p.threads, (int32_t)p.blobBytes, (int32_t)list.size()};
         std::copy(v, v + 6, info);
         for (size_t k = 0; k < list.size() && (int)k < maxSteps; k++) {
             const int32_t f[6] = {list[k].op, list[k].level, list[k].from, list[k].to, list[k].clusterWide, list[k].flag};
