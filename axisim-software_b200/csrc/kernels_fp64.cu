@@ -1152,8 +1152,10 @@ __device__ __forceinline__ double caseLane(const double* __restrict__ x, int n, 
     for (; n < n1; n += kCaseAhead * kThreads) {
         double v[kCaseAhead];
 #pragma unroll
-        for (int k = 0; k < kCaseAhead; k++) v[k] = n + k * kThreads < n1 ? fabs(x[n + k * kThreads]) : 0.0;
-        // a lane's surplus values are +0: they change neither a sum of absolute values nor their maximum
+        for (int k = 0; k < kCaseAhead; k++)
+            v[k] = n + k * kThreads < n1 ? fabs(x[n + k * kThreads]) : MAX ? -INFINITY : 0.0;
+        // surplus values change neither a sum of absolute values (+0) nor a
+        // maximum, which stays empty where every value is a NaN (-inf)
 #pragma unroll
         for (int k = 0; k < kCaseAhead; k++) acc = combine(acc, SQUARE ? v[k] * v[k] : v[k], MAX);
     }
