@@ -2843,9 +2843,7 @@ int Solver::solve(int continueRun, axisim_result* res) {
                 CK(cudaMemcpyAsync(b.old(), b.phi, (size_t)N_ * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
             }
         }
-        // the first iteration of a step is decided here, each later one by the
-        // end of the one before it (k_iter_end)
-        h.done = __atomic_load_n(hostStop_, __ATOMIC_SEQ_CST) ? 2 : 0;
+        h.done = 0;
         h.checked = 1;
         h.k = 0;
         h.bdf2 = (bdf2 && t > 0) ? 1 : 0;
@@ -2856,7 +2854,15 @@ int Solver::solve(int continueRun, axisim_result* res) {
         int batch = 4;
         int launched = 0;
         int drained = 0;
-        while (!h.done) {
+        for (;;) {
+            // each iteration's end decides about the next one (k_iter_end); the first
+            // one of a batch is decided here: a stop requested since, by the residual
+            // callback for one
+            if (!h.done && __atomic_load_n(hostStop_, __ATOMIC_SEQ_CST)) {
+                h.done = 2;
+                CK(cudaMemcpyAsync(ctl_, &h, sizeof(Ctl), cudaMemcpyHostToDevice, stream_));
+            }
+            if (h.done) break;
             const int nb = std::min(batch, std::max(1, csim_.maxIter - launched));
             for (int i = 0; i < nb; i++) CK(cudaGraphLaunch(exec_, stream_));
             launched += nb;
