@@ -37,7 +37,8 @@ constexpr int kThreads = 256;
 constexpr int kQ = 5;  // stat_u, scale_u, stat_v, scale_v, continuity
 constexpr int kMaxBlocks = AXISIM_STATIC_MAX_CELLS / kThreads;
 constexpr int kPartialDoubles = kMaxBlocks * kQ;
-constexpr int kWordDoubles = 32;  // 256 bytes of counters after the partials
+constexpr int kCallSlots = 256;         // calls take them in turn
+constexpr int kWordDoubles = kCallSlots + 2;  // a slot's two counters (8 bytes) each, after the partials
 constexpr int kMaxDevices = 64;
 constexpr int kResident = 148 * 4;  // blocks that run at once (64 registers a thread)
 constexpr int kMaxGroups = 28;      // groups a block: kMaxBlocks over kResident
@@ -45,9 +46,12 @@ constexpr int kMaxGroups = 28;      // groups a block: kMaxBlocks over kResident
 static_assert(AXISIM_STATIC_MAX_CELLS % kThreads == 0, "limit must be whole blocks");
 static_assert(kMaxGroups * kResident >= kMaxBlocks, "every group has a block");
 
-// Partials of up to kMaxBlocks blocks, then the counters: [0] arrival ticket,
-// [1] number of cells that met an out-of-range index, both zero between calls,
-// [2] the last call's count. 640 KiB + 256 B per device.
+// Partials of up to kMaxBlocks blocks, then two counters per call slot: the
+// arrival ticket and the number of cells that met an out-of-range index. The
+// last block of a call returns its slot's counters to zero, and only that
+// call's blocks touch them, so calls that overlap in time, whose sums may be
+// wrong, leave nothing behind. The last two words hold the count of the call
+// that has no host word. 640 KiB + 2 KiB per device.
 static __device__ __align__(256) double g_residualScratch[kPartialDoubles + kWordDoubles];
 
 __device__ __forceinline__ double combine(double a, double b, int isMax) { return isMax ? fmax(a, b) : a + b; }
@@ -60,8 +64,7 @@ k_residual_static(int N, int F, int S, const int32_t* __restrict__ cellFaceStart
                   const double* __restrict__ bv, const double* __restrict__ u, const double* __restrict__ v,
                   const double* __restrict__ mDot, int normU, int normV, double* __restrict__ resU,
                   double* __restrict__ resV, double* __restrict__ resC, double* __restrict__ sums,
-                  double* scratch, int wide, int groups, volatile unsigned int* status) {
-    unsigned int* words = reinterpret_cast<unsigned int*>(scratch + kPartialDoubles);
+                  double* scratch, unsigned int* words, int wide, int groups, volatile unsigned int* status) {
     const int isMax[kQ] = {normU == 2, 0, normV == 2, 0, 0};
     // groups of 256 cells, several a block: one arrival for all of them
     __shared__ double sh[kMaxGroups][kThreads / 32][kQ];
@@ -198,24 +201,25 @@ k_residual_static(int N, int F, int S, const int32_t* __restrict__ cellFaceStart
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int q = 0; q < kQ; q++) sums[q] = tr[0][q];
-        // the counters return to zero for the next call
-        const unsigned int bad = words[1];
-        if (status) *status = bad;
-        else words[2] = bad;
+        // the counters return to zero for the slot's next call
+        *status = words[1];
         words[1] = 0u;
         words[0] = 0u;
     }
 }
 
-// Per-device address of the scratch array, looked up once per device.
+// Per-device address of the scratch array, looked up once per device, and the
+// calls' turns at its slots.
 std::mutex g_setupMu;
 double* g_scratchPtr[kMaxDevices] = {};
-// A page-locked host word per device for a call's bad-index count, mapped into
-// the device (host memory, taken on the first call): the kernel's own store
-// saves the copy back, some 10 of 39 us of a small call. Null where it could not
-// be had: the count is then copied from the scratch words.
-volatile unsigned int* g_status[kMaxDevices] = {};
+unsigned int g_calls[kMaxDevices] = {};
+// A page-locked host word per call slot and device for a call's bad-index count,
+// mapped into the device (host memory, taken on the first call): the kernel's own
+// store saves the copy back, some 10 of 39 us of a small call. Null where it
+// could not be had: the count is then copied from the scratch words.
+volatile unsigned int* g_status = nullptr;
 bool g_statusTried = false;
+constexpr unsigned int kUnwritten = 0xFFFFFFFFu;  // no count: at most one a cell
 
 void setError(char* err, size_t errLen, const char* msg) {
     if (!err || errLen == 0) return;
@@ -287,7 +291,8 @@ extern "C" int axisim_residual_static(int32_t nCells, int32_t nFaces, int32_t nS
         return AXISIM_E_ARG;
     }
     double* scratch = nullptr;
-    volatile unsigned int* status = nullptr;
+    volatile unsigned int* hostWord = nullptr;
+    unsigned int slot = 0;
     {
         std::lock_guard<std::mutex> lk(g_setupMu);
         if (!g_scratchPtr[dev]) {
@@ -303,16 +308,17 @@ extern "C" int axisim_residual_static(int32_t nCells, int32_t nFaces, int32_t nS
         if (!g_statusTried) {
             g_statusTried = true;
             void* p = nullptr;
-            if (cudaHostAlloc(&p, sizeof(unsigned int) * 64 * kMaxDevices, cudaHostAllocPortable | cudaHostAllocMapped) ==
-                cudaSuccess)
-                for (int d = 0; d < kMaxDevices; d++)  // a word in a line of its own
-                    g_status[d] = static_cast<volatile unsigned int*>(p) + 64 * d;
+            if (cudaHostAlloc(&p, sizeof(unsigned int) * kCallSlots * kMaxDevices,
+                              cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
+                g_status = static_cast<volatile unsigned int*>(p);
             cudaGetLastError();
         }
-        status = g_status[dev];
+        slot = g_calls[dev]++ % kCallSlots;
+        if (g_status) hostWord = g_status + (size_t)dev * kCallSlots + slot;
     }
-    unsigned int* words = reinterpret_cast<unsigned int*>(scratch + kPartialDoubles);
-    // the arrival ticket and the bad-index count are zero between calls
+    unsigned int* words = reinterpret_cast<unsigned int*>(scratch + kPartialDoubles) + 2 * slot;
+    unsigned int* devWord = reinterpret_cast<unsigned int*>(scratch + kPartialDoubles) + 2 * kCallSlots;
+    if (hostWord) *hostWord = kUnwritten;
     {
         const int nGroups = (nCells + kThreads - 1) / kThreads;
         const int groups = std::min(kMaxGroups, (nGroups + kResident - 1) / kResident);
@@ -321,16 +327,21 @@ extern "C" int axisim_residual_static(int32_t nCells, int32_t nFaces, int32_t nS
         const int wide = ((reinterpret_cast<uintptr_t>(cellFaceIDs) | reinterpret_cast<uintptr_t>(AF)) & 15) == 0;
         k_residual_static<<<blocks, kThreads, 0, s>>>(nCells, nFaces, nSlots, cellFaceStart, cellFaceIDs, faceOwner,
                                                       faceNeighbor, AF, ACu, ACv, bu, bv, u, v, mDot, normU, normV,
-                                                      resU, resV, resC, sums, scratch, wide, groups, status);
+                                                      resU, resV, resC, sums, scratch, words, wide, groups,
+                                                      hostWord ? hostWord : devWord);
         e = cudaGetLastError();
     }
     unsigned int bad = 0;
-    if (e == cudaSuccess && !status) e = cudaMemcpyAsync(&bad, words + 2, sizeof bad, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && !hostWord) e = cudaMemcpyAsync(&bad, devWord, sizeof bad, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess && status) bad = *status;
+    if (e == cudaSuccess && hostWord) bad = *hostWord;
     if (e != cudaSuccess) {
         std::snprintf(msg, sizeof msg, "CUDA: %s", cudaGetErrorString(e));
         setError(err, errLen, msg);
+        return AXISIM_E_CUDA;
+    }
+    if (bad == kUnwritten) {  // more calls at once than slots
+        setError(err, errLen, "too many calls overlapped: the results were not written");
         return AXISIM_E_CUDA;
     }
     if (bad) {

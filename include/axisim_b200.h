@@ -497,7 +497,7 @@ int axisim_mesh_segments(axisim_handle* h, int32_t* nSegments, int32_t* nOffsetS
  * allocation: for callers that cannot allocate at that point -- a host whose
  * GPU memory is all held by another allocator or capped, or a monitoring hook
  * inside a time-critical loop where cudaMalloc/cudaFree would stall the device.
- * The first call of a process page-locks 16 KB of host memory for the status.
+ * The first call of a process page-locks 64 KB of host memory for the status.
  * The reduction scratch is a fixed file-scope device array sized for at most
  * AXISIM_STATIC_MAX_CELLS cells; larger nCells is rejected with AXISIM_E_ARG.
  * Inputs, all device pointers on the current device, in the reference's CSR
@@ -517,7 +517,7 @@ int axisim_mesh_segments(axisim_handle* h, int32_t* nSegments, int32_t* nOffsetS
  * into another GPU's memory are rejected (AXISIM_E_ARG). Out-of-range indices
  * are skipped and reported as AXISIM_E_MESH with their count. All calls share
  * the scratch: calls that overlap in time (other threads, or other streams
- * still running) race and give wrong sums.
+ * still running) race and give wrong sums; a later call on its own is not affected.
  * Messages go to err[errLen] (may be NULL). */
 #define AXISIM_STATIC_MAX_CELLS 4194304
 int axisim_residual_static(int32_t nCells, int32_t nFaces, int32_t nSlots, const int32_t* cellFaceStart,
