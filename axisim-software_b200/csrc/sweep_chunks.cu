@@ -20,8 +20,8 @@
 // The arithmetic and its order are those of the per-sweep kernels
 // (k_jacobi_uv, k_gs_uv, k_jacobi1, k_gs1, k_jacobi_uv32;
 // linear_solver.cu:9-72), so the results are the same bit for bit. An unused
-// slot has the coefficient +0 (-0 in the FP32 form, which subtracts by one
-// rounding) and reads a zero cell: it changes no sum. Compiled with --fmad=false.
+// slot has the coefficient +0 and reads a zero cell: the sum less +0, or in the
+// FP32 form -0 times 0 plus the sum, is the sum. Compiled with --fmad=false.
 #include <algorithm>
 
 #include <cooperative_groups.h>
@@ -149,14 +149,15 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_sweep_chunks(const Ctl* ct
         // the other iterate and no halo; a colour's rows arrive in cells that
         // rows of the same colour do not read.
         sweepRows(I.start[k], I.boundary[k], MODE == kCluster && more);
-        if (MODE == kCluster && more) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        // a warp's lanes come from loops of different lengths: the barrier's unaligned form
+        if (MODE == kCluster && more) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
         sweepRows(I.boundary[k], I.start[k + 1], false);
         if (!colors) {
             V* t = x;
             x = y;
             y = t;
         }
-        if (MODE == kCluster && more) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (MODE == kCluster && more) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
         __syncthreads();
     }
     // the result, in place of the start: two steps or more, so every CTA that
