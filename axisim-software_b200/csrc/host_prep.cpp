@@ -841,9 +841,8 @@ void coarseMembers(const GridLevel& fine, const GridLevel& coarse, std::vector<i
         if (fine.cellToCoarse[(size_t)n] >= 0) list[(size_t)fill[(size_t)fine.cellToCoarse[(size_t)n]]++] = n;
 }
 
-// The cells along a Morton curve of their centres: exact within buckets of more
-// than `refine` cells, by cell id within smaller ones.
-static std::vector<int32_t> curveOrder(int N, const double* cz, const double* cr, int refine) {
+// The cells' keys along a Morton curve of their centres (one scale for both axes).
+static std::vector<uint32_t> curveKeys(int N, const double* cz, const double* cr) {
     double z0 = cz[0], z1 = cz[0], r0 = cr[0], r1 = cr[0];
     for (int n = 1; n < N; n++) {
         z0 = std::min(z0, cz[n]);
@@ -862,6 +861,30 @@ static std::vector<int32_t> curveOrder(int N, const double* cz, const double* cr
             key[(size_t)n] = spreadBits16(iz) | (spreadBits16(ir) << 1);
         }
     });
+    return key;
+}
+
+// The cells along the curve, by cell id within a key: three counting passes on
+// one thread, which some ten thousand cells take in the time that the passes
+// below spend on their 65,536 buckets.
+static std::vector<int32_t> smallCurveOrder(int N, const double* cz, const double* cr) {
+    const std::vector<uint32_t> key = curveKeys(N, cz, cr);
+    std::vector<int32_t> order((size_t)N), next((size_t)N);
+    std::iota(order.begin(), order.end(), 0);
+    for (int shift = 0; shift < 32; shift += 11) {
+        int32_t at[2049] = {};
+        for (int n = 0; n < N; n++) at[(key[(size_t)n] >> shift & 2047u) + 1]++;
+        for (int d = 0; d < 2048; d++) at[d + 1] += at[d];
+        for (int n : order) next[(size_t)at[key[(size_t)n] >> shift & 2047u]++] = n;
+        order.swap(next);
+    }
+    return order;
+}
+
+// The same curve: exact within buckets of more than `refine` cells, by cell id
+// within smaller ones.
+static std::vector<int32_t> curveOrder(int N, const double* cz, const double* cr, int refine) {
+    const std::vector<uint32_t> key = curveKeys(N, cz, cr);
     // cells by key: a counting sort on the top 16 bits (a 256 x 256 grid of
     // the bounding square; per-thread counts, so each bucket keeps ascending
     // cell order), then large buckets by the whole key
@@ -971,56 +994,52 @@ SweepTiles buildSweepTiles(int N, int W, const int32_t* nb, const double* cz, co
 SweepChunks buildSweepChunks(int N, int W, const int32_t* nb, const double* cz, const double* cr, int chunks,
                              const int32_t* color, int nColors) {
     SweepChunks t;
-    if (N <= 0 || W < 1 || W > 4 || chunks < 1 || chunks > 1024 || nColors < 1 || nColors > SweepChunks::kMaxColors)
+    if (N <= 0 || W < 3 || W > 4 || chunks < 1 || chunks > SweepChunks::kMaxChunks || nColors < 1 ||
+        nColors > SweepChunks::kMaxColors)
         return t;
     const int per = (N + chunks - 1) / chunks;
     chunks = (N + per - 1) / per;
     if (per >= 0x7000) return t;
-    t.cells = chunks > 1 ? curveOrder(N, cz, cr, std::max(32, per / 8)) : std::vector<int32_t>();
+    t.cells = chunks > 1 ? smallCurveOrder(N, cz, cr) : std::vector<int32_t>();
     if (chunks == 1) {
         t.cells.resize((size_t)N);
         for (int n = 0; n < N; n++) t.cells[(size_t)n] = n;
     }
     t.info.resize((size_t)chunks);
     std::vector<int16_t> chunkOf((size_t)N);
-    parallelFor(chunks, [&](int c0, int c1) {
-        for (int c = c0; c < c1; c++)
-            for (int p = c * per, e = std::min(N, p + per); p < e; p++) chunkOf[(size_t)t.cells[(size_t)p]] = (int16_t)c;
-    }, 4);
-    // rows of a chunk: by colour, within it those that other chunks read first, then by cell
-    std::vector<int32_t> posOf((size_t)N);  // position of a cell in t.cells
-    std::vector<char> exported((size_t)N);
-    parallelFor(chunks, [&](int c0, int c1) {
-        for (int c = c0; c < c1; c++) {
-            SweepChunks::Info& I = t.info[(size_t)c];
-            I.row0 = c * per;
-            I.rows = std::min(N, I.row0 + per) - I.row0;
-            int32_t* b = t.cells.data() + I.row0;
-            for (int i = 0; i < I.rows; i++) {
-                const int n = b[i];
-                char x = 0;
-                for (int j = 0; j < W; j++) {
-                    const int m = nb[(size_t)j * N + n];
-                    if (m >= 0 && chunkOf[(size_t)m] != c) x = 1;
-                }
-                exported[(size_t)n] = x;
-            }
-            auto rank = [&](int n) { return 2 * (color ? color[n] : 0) + (exported[(size_t)n] ? 0 : 1); };
-            std::sort(b, b + I.rows, [&](int32_t x, int32_t y) {
-                const int rx = rank(x), ry = rank(y);
-                return rx != ry ? rx < ry : x < y;
-            });
-            int at = 0;
-            for (int k = 0; k < nColors; k++) {
-                I.start[k] = at;
-                while (at < I.rows && rank(b[at]) == 2 * k) at++;
-                I.boundary[k] = at;
-                while (at < I.rows && rank(b[at]) == 2 * k + 1) at++;
-            }
-            I.start[nColors] = at;
-            for (int i = 0; i < I.rows; i++) posOf[(size_t)b[i]] = I.row0 + i;
+    for (int p = 0; p < N; p++) chunkOf[(size_t)t.cells[(size_t)p]] = (int16_t)(p / per);
+    // rows of a chunk: by colour, within it those that other chunks read first,
+    // then by cell: the cells in order, counted into their chunk's ranks
+    const int ranks = 2 * nColors;
+    std::vector<uint8_t> rank((size_t)N);
+    std::vector<int32_t> at((size_t)chunks * ranks + 1, 0);
+    for (int n = 0; n < N; n++) {
+        bool exported = false;
+        for (int j = 0; j < W; j++) {
+            const int m = nb[(size_t)j * N + n];
+            exported = exported || (m >= 0 && chunkOf[(size_t)m] != chunkOf[(size_t)n]);
         }
-    }, 4);
+        rank[(size_t)n] = (uint8_t)(2 * (color ? color[n] : 0) + (exported ? 0 : 1));
+        at[(size_t)chunkOf[(size_t)n] * ranks + rank[(size_t)n] + 1]++;
+    }
+    for (size_t k = 1; k < at.size(); k++) at[k] += at[k - 1];
+    for (int c = 0; c < chunks; c++) {
+        SweepChunks::Info& I = t.info[(size_t)c];
+        const int32_t* first = at.data() + (size_t)c * ranks;
+        I.row0 = first[0];
+        I.rows = first[ranks] - first[0];
+        for (int k = 0; k < nColors; k++) {
+            I.start[k] = first[2 * k] - first[0];
+            I.boundary[k] = first[2 * k + 1] - first[0];
+        }
+        I.start[nColors] = I.rows;
+    }
+    std::vector<int32_t> posOf((size_t)N);  // position of a cell in t.cells
+    for (int n = 0; n < N; n++) {
+        const int p = at[(size_t)chunkOf[(size_t)n] * ranks + rank[(size_t)n]]++;
+        t.cells[(size_t)p] = n;
+        posOf[(size_t)n] = p;
+    }
     // halos, then the rows' local references
     std::vector<std::vector<int32_t>> halo((size_t)chunks);
     t.ref.assign(4 * (size_t)N, 0);

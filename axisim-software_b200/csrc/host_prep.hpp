@@ -162,11 +162,11 @@ SweepTiles buildSweepTiles(int nCells, int W, const int32_t* nb, const double* c
 // The mesh in `chunks` pieces of equal size along a curve of the cell centres,
 // for linear sweeps that stay on the chip (sweep_chunks.cu): a piece's rows by
 // colour, those that other pieces read first, and its halo, the cells of other
-// pieces that its rows refer to. nb is the slot neighbour block [W][N], W <= 4;
+// pieces that its rows refer to. nb is the slot neighbour block [W][N], W 3 or 4;
 // color (null: one colour) orders Gauss-Seidel sweeps. No pieces when they do
 // not fit 15-bit local references.
 struct SweepChunks {
-    static constexpr int kMaxColors = 8;
+    static constexpr int kMaxColors = 8, kMaxChunks = 16;
     struct Info {
         int32_t row0 = 0, rows = 0, halo0 = 0, halos = 0, push0 = 0, pushes = 0;
         int32_t start[kMaxColors + 1] = {};  // first row of each colour (and the end)

@@ -1333,6 +1333,7 @@ private:
         std::vector<unsigned char> blob;
         cluster_ = findClusterPlan(hier_, lastTerminal, sliceOffH, mStartH, mListH, blob);
         if (cluster_.first >= 0 && !clusterRunnable(cluster_)) cluster_ = MgClusterPlan();
+        if (cluster_.first >= 0) mgArena_.reserve(blob.size());  // not the arena's next, larger chunk for it alone
         if (cluster_.first >= 0) cluster_.blob = mgArena_.upload(blob.data(), blob.size());
     }
     int tailStart_ = -1;
@@ -1447,7 +1448,10 @@ private:
                     std::copy(f.start, f.start + 9, o.start);
                     std::copy(f.boundary, f.boundary + 8, o.boundary);
                 }
+                // one small allocation: the driver has room for it in a block it holds
                 Arena& A = chunkArena_;
+                A.reserve(info.size() * sizeof info[0] + (t.cells.size() + t.halo.size() + t.pushAt.size()) * sizeof(int32_t) +
+                          t.ref.size() * sizeof(uint16_t) + t.push.size() * sizeof(uint32_t) + 6 * 256);
                 d.info = A.upload(info.data(), info.size());
                 d.cells = A.upload(t.cells.data(), t.cells.size());
                 d.halo = A.upload(t.halo.data(), t.halo.size());
