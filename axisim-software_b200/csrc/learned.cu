@@ -1799,13 +1799,15 @@ void LearnedNet::trainStep(const Sample& smp, float lr, int t, float* lossOut, c
     lossAndGrad(smp, lossOut, s);
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)t), c2 = 1.f - std::pow(b2, (float)t);
-    if (wBf16_)
-        launchPDL(k_adam<bfloat>, dim3(blocksFor(nParams_)), dim3(kThreads), 0, s, nParams_, params_, grad_, adamM_, adamV_,
-                                                                (bfloat*)paramsLow_, lr, b1, b2, 1e-8f, c1, c2);
-    if (wBf16_) packWeights(s);
-    else
-        launchPDL(k_adam<float>, dim3(blocksFor(nParams_)), dim3(kThreads), 0, s, nParams_, params_, grad_, adamM_, adamV_, params_, lr,
-                                                               b1, b2, 1e-8f, c1, c2);
+    const dim3 grid(blocksFor(nParams_)), block(kThreads);
+    if (wBf16_) {
+        launchPDL(k_adam<bfloat>, grid, block, 0, s, nParams_, params_, grad_, adamM_, adamV_, (bfloat*)paramsLow_, lr,
+                  b1, b2, 1e-8f, c1, c2);
+        packWeights(s);
+    } else {
+        launchPDL(k_adam<float>, grid, block, 0, s, nParams_, params_, grad_, adamM_, adamV_, params_, lr, b1, b2,
+                  1e-8f, c1, c2);
+    }
     NCK(cudaGetLastError());
 }
 

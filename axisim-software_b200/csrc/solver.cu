@@ -1409,8 +1409,8 @@ private:
     // meshes keep a launch per sweep. Whole 20-iteration runs, on chip against a
     // launch per sweep: 13.7k cells 3.87 / 4.19 ms FP64, 3.60 / 3.78 mixed; 28k
     // cells 4.36 / 4.53 and 3.96 / 4.10; 53k cells 9.04 / 8.62 (mixed, 40
-    // iterations): 16 SMs become the bound, and the pieces take the host 60 us per
-    // thousand cells, so the line is where it pays within some 50 iterations.
+    // iterations): 16 SMs become the bound, and the pieces take the host 45 us per
+    // thousand cells on a first solve, which some ten iterations at the line save.
     static constexpr int kSweepCtaCells = 2048;
     static constexpr int kSweepClusterCells = 16384;
     void ensureSweepChunks() {

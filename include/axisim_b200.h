@@ -348,7 +348,10 @@ int axisim_learned_grad(axisim_handle* h, int32_t sample, float* loss, float* gr
 int axisim_learned_train(axisim_handle* h, int32_t steps, float lr, uint64_t seed, int32_t first, int32_t count,
                          float* lossOut);
 /* The network's correction out[nCells] (its output times rms(r / A_C)) for a
- * residual r, A_C diagonal and boundary deficit (host arrays). */
+ * residual r, A_C diagonal and boundary deficit (host arrays). With BF16 weights
+ * its sums run in another order than those of the pass that a solve applies and
+ * a loss is formed on: the outputs differ by FP32 roundings (some 1e-6
+ * relative), with BF16 activations by roundings of those. */
 int axisim_learned_predict(axisim_handle* h, const float* r, const float* acDiag, const float* deficit, float* out);
 /* AXISIM_LEARNED_*; takes effect in the FCG pressure solver. */
 int axisim_learned_enable(axisim_handle* h, int32_t mode);
