@@ -1255,8 +1255,9 @@ inline bool slabs(const NetLayer& L) {
 // and 2.08 with four on every level).
 inline int mmaBlocks(int cols) { return std::min(cols / 8, 8); }
 
-// One wave of CTAs that loop over the tiles: as many as shared memory (192 KB
-// of weights an SM) and 48 warps an SM allow.
+// CTAs that loop over the tiles: at most as many as shared memory (192 KB of
+// weights an SM) and 48 warps an SM would hold. Their registers (127) let 16
+// warps an SM run at once; a grid of just those measured the same.
 inline int mmaCtas(const NetLayer& L, int tilesPerCta, size_t smem) {
     const int perSm = (int)std::min<size_t>(48 * 32 / kMmaThreads, 192 * 1024 / smem);
     return std::min((L.N + 16 * tilesPerCta - 1) / (16 * tilesPerCta), 148 * perSm);
