@@ -2,7 +2,8 @@
 whose cases' coarsest levels, merged, are larger than it has threads: every case
 equals its standalone solve bit for bit, in FP64 and mixed precision, on both
 sides of 512 and of 1,024 rows. Small cases that share one hierarchy, with whole
-slices of isolated coarse cells: the oracle's fields bit for bit.
+slices of isolated coarse cells, and meshes with a single coarse level: the
+oracle's fields bit for bit.
 """
 import numpy as np
 import pytest
@@ -54,6 +55,24 @@ def test_isolated_cells_match_the_oracle(name):
     gpu = abi.Solver(union, bcs, members[0].settings)
     gpu.solve()
     orc = oracle.Oracle(union, bcs, members[0].settings)
+    orc.run()
+    for f in FIELDS + ("pp",):
+        np.testing.assert_array_equal(gpu.get(f), orc.get(f), err_msg=f)
+    gpu.close()
+    orc.close()
+
+
+@pytest.mark.parametrize("coarse", [0, 1, 2, 30])
+@pytest.mark.parametrize("nr,nz", [(8, 16), (10, 10), (5, 37)])
+def test_a_single_coarse_level_matches_the_oracle(nr, nz, coarse):
+    c = _member(0, nr, nz)
+    c.settings.update(mgLinearSweep=coarse)
+    mesh = abi.multiblock(c.blocks)
+    plan = abi.vcycle_cluster_host(mesh, coarse=coarse)
+    assert (plan["first"], plan["count"]) == (1, 1)
+    gpu = abi.Solver(mesh, c.bc_fields(), c.settings)
+    gpu.solve()
+    orc = oracle.Oracle(mesh, c.bc_fields(), c.settings)
     orc.run()
     for f in FIELDS + ("pp",):
         np.testing.assert_array_equal(gpu.get(f), orc.get(f), err_msg=f)
